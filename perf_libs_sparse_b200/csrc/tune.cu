@@ -83,7 +83,23 @@ void apply_config(Mat *A, const SpmvConfig &cfg) {
     // Spread chunks much wider than the typical one over several lane
     // groups (power-law row lengths).
     const double mean_w = A->sell.nC ? (double)A->sell.size / (A->sell.nC * (double)c.C) : 0;
-    const int slice = std::max(64, (int)std::ceil(mean_w * 8));
+    // Slice width. A launch lasts at least as long as one lane group's walk
+    // along its widest unsliced chunk (two slices), about 0.2 us a column
+    // under load, so the slices get narrower with the matrix: about a quarter
+    // of the launch (size elements at some 200 a nanosecond) for that walk,
+    // i.e. size >> 19 columns, but at least 2 mean widths (32 columns), below
+    // which the partial sums and counts cost more than the walk, and at most 8
+    // mean widths (64 columns), past which a large matrix gains nothing.
+    // Measured on power-law rows of mean 16 (C = 16, sigma = 8192, us; 8 mean
+    // widths -> this rule): n = 30,000 77 -> 21, 150,000 100 -> 27, 1 M
+    // 127 -> 80, 4.2 M 314 -> 315 (32 columns there: 343).
+    const int widest = std::max(64, (int)std::ceil(mean_w * 8));
+    int slice = std::max<int>({32, (int)std::ceil(mean_w * 2), (int)(A->sell.size >> 19)});
+    slice = std::min(widest, (slice + 3) / 4 * 4);
+    // Below the 8 mean widths a slice holds at least size / 2^19 columns and a
+    // sliced chunk more than 2 slices, so the slots (at most 1.5 per slice of
+    // a chunk's width) times C stay under 1.5 * 2^19, inside the 2^21 partial
+    // sums of the allocation-free entry point.
     if (A->sell.max_width > 4 * slice)
       sell_build_work_list(A->sell, slice, s);
     else

@@ -238,7 +238,8 @@ perflibs_status_t create_csr(Mat **out, int32_t m, int32_t n, const int32_t *row
     upload(c.vals, vals, sizeof(T) * A->nnz, s);
     // Indices are checked before any kernel uses them (the reference reads
     // them as they are).
-    const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(), s);
+    const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(),
+                                      s, &c.max_row);
     if (bad.first >= 0)
       return param_error(A, 4, "row_ptr decreases or leaves [0, nnz] at row " + std::to_string(bad.first));
     if (bad.second >= 0)
@@ -1363,11 +1364,7 @@ void run_spmv(Mat *A, int op, const X *x, X *y, X alpha, X beta, cudaStream_t s)
     }
   }
   if (A->has_csrT && A->csrT.lo == A->csr.lo) {
-    const double mean = A->n > 0 ? (double)A->csrT.nnz / A->n : 1;
-    int tpr = 1;
-    while (tpr * 2 <= mean && tpr < 32)
-      tpr *= 2;
-    spmv_csr<X>(A->csrT, A->n, tpr, x, y, alpha, beta, s);
+    spmv_csr<X>(A->csrT, A->n, csr_lanes(A->csrT, A->n), x, y, alpha, beta, s);
   } else {
     spmv_csr_trans<X>(A->csr, A->m, A->n, x, y, alpha, beta, s);
   }
@@ -2238,7 +2235,8 @@ perflibs_status_t perflibs_b200_spmat_create_csr_d_dev(perflibs_spmat_t *out, in
         k_sub_base<<<(unsigned)div_up(A->nnz, 256), 256, 0, s>>>(A->nnz, 1, c.col.as<int32_t>());
       PLS_LAUNCH_CHECK();
     }
-    const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(), s);
+    const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(),
+                                      s, &c.max_row);
     if (bad.first >= 0)
       return param_error(A, 4, "row_ptr decreases or leaves [0, nnz] at row " + std::to_string(bad.first));
     if (bad.second >= 0)

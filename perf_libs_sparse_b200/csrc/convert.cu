@@ -364,6 +364,33 @@ void convert_values(const void *in, Vt vin, void *out, Vt vout, int64_t n,
   PLS_LAUNCH_CHECK();
 }
 
+namespace {
+
+__global__ void k_longest_row(int32_t m, const int32_t *__restrict__ rp,
+                              int32_t *__restrict__ out) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int len = __reduce_max_sync(0xffffffffu, r < m ? rp[r + 1] - rp[r] : 0);
+  if (len > 0 && (threadIdx.x & 31) == 0)
+    atomicMax(out, len);
+}
+
+// The longest row of a CSR matrix the library made itself.
+void record_longest_row(CsrDev &c, int32_t m, cudaStream_t s) {
+  c.max_row = 0;
+  if (m <= 0 || c.nnz == 0)
+    return;
+  DevBuf out;
+  out.reserve(4);
+  PLS_CUDA(cudaMemsetAsync(out.p, 0, 4, s));
+  k_longest_row<<<(unsigned)div_up(m, 256), 256, 0, s>>>(m, c.row_ptr.as<int32_t>(),
+                                                         out.as<int32_t>());
+  PLS_LAUNCH_CHECK();
+  PLS_CUDA(cudaMemcpyAsync(&c.max_row, out.p, 4, cudaMemcpyDeviceToHost, s));
+  PLS_CUDA(cudaStreamSynchronize(s));
+}
+
+}  // namespace
+
 void build_csr_transpose(const CsrDev &c, int32_t m, int32_t n, CsrDev &out,
                          cudaStream_t s) {
   CsrDev T;
@@ -416,6 +443,7 @@ void build_csr_transpose(const CsrDev &c, int32_t m, int32_t n, CsrDev &out,
     PLS_LAUNCH_CHECK();
     PLS_CUDA(cudaStreamSynchronize(s));
   }
+  record_longest_row(T, n, s);
   out = std::move(T);
 }
 
@@ -457,13 +485,20 @@ namespace {
 __global__ void k_check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                    const int32_t *__restrict__ ptr,
                                    const int32_t *__restrict__ idx,
-                                   unsigned long long *__restrict__ bad) {
+                                   unsigned long long *__restrict__ bad,
+                                   unsigned *__restrict__ longest) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int32_t len = 0;
   if (i < rows) {
     const int32_t a = ptr[i], b = ptr[i + 1];
     if (a < 0 || b < a || b > nnz)
       atomicMin(bad, (unsigned long long)i);
+    else
+      len = b - a;
   }
+  len = __reduce_max_sync(0xffffffffu, len);
+  if (len > 0 && (threadIdx.x & 31) == 0)
+    atomicMin(longest, ~(unsigned)len);  // all ones before the first
   if (i < nnz) {
     const int32_t c = idx[i];
     if (c < 0 || c >= cols)
@@ -476,22 +511,26 @@ __global__ void k_check_compressed(int32_t rows, int32_t cols, int64_t nnz,
 // Structure check of 0-based compressed arrays before any kernel indexes
 // with them: the first row whose pointers are decreasing or outside
 // [0, nnz], and the first entry whose index is outside [0, cols); -1 each
-// when there is none.
+// when there is none. On the way, the longest row.
 std::pair<int64_t, int64_t> check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                              const int32_t *ptr, const int32_t *idx,
-                                             cudaStream_t s) {
+                                             cudaStream_t s, int32_t *longest) {
+  if (longest)
+    *longest = 0;
   const int64_t work = std::max<int64_t>(rows, nnz);
   if (work == 0)
     return {-1, -1};
   DevBuf bad;
-  bad.reserve(16);
-  PLS_CUDA(cudaMemsetAsync(bad.p, 0xff, 16, s));
+  bad.reserve(24);
+  PLS_CUDA(cudaMemsetAsync(bad.p, 0xff, 24, s));
   k_check_compressed<<<(unsigned)div_up(work, 256), 256, 0, s>>>(
-      rows, cols, nnz, ptr, idx, bad.as<unsigned long long>());
+      rows, cols, nnz, ptr, idx, bad.as<unsigned long long>(), bad.as<unsigned>() + 4);
   PLS_LAUNCH_CHECK();
-  unsigned long long h[2];
-  PLS_CUDA(cudaMemcpyAsync(h, bad.p, 16, cudaMemcpyDeviceToHost, s));
+  unsigned long long h[3];
+  PLS_CUDA(cudaMemcpyAsync(h, bad.p, 24, cudaMemcpyDeviceToHost, s));
   PLS_CUDA(cudaStreamSynchronize(s));
+  if (longest)
+    *longest = (int32_t) ~(unsigned)h[2];
   return {h[0] == ~0ull ? -1 : (int64_t)h[0], h[1] == ~0ull ? -1 : (int64_t)h[1]};
 }
 
@@ -560,6 +599,7 @@ int64_t coo_to_csr(int32_t m, int32_t n, int64_t nnz, const int32_t *row, const 
     PLS_LAUNCH_CHECK();
   }
   PLS_CUDA(cudaStreamSynchronize(s));
+  record_longest_row(R, m, s);
   out = std::move(R);
   return -1;
 }
@@ -604,6 +644,7 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
   });
   PLS_LAUNCH_CHECK();
   PLS_CUDA(cudaStreamSynchronize(s));
+  record_longest_row(R, m, s);
   out = std::move(R);
 }
 

@@ -378,6 +378,7 @@ struct CsrDev {
   int64_t nnz = 0;
   uint64_t vals_version = 0;  // counts value updates (invalidates value copies)
   int32_t ncols = 0;  // columns (bound of col); 0 when not recorded
+  int32_t max_row = INT32_MAX;  // longest row; INT32_MAX when not recorded
   Vt vt = Vt::F64;
   // Reduced-precision copy of the values used by the kernels when the
   // handle's storage mode asks for one.
@@ -559,6 +560,14 @@ cudaStream_t stream_of(const Mat *A);
 template <class X>
 void spmv_csr(const CsrDev &c, int32_t m, int tpr, const X *x, X *y, X alpha,
               X beta, cudaStream_t s);
+// CSR vector kernel: entries a lane loads together with `lanes` lanes per
+// row, and the row length past which the whole warp takes the row (more than
+// kCsrLongGroups round trips of its lanes).
+constexpr int kCsrLongGroups = 4;
+constexpr int csr_group(int lanes) { return lanes == 1 ? 8 : 4; }
+constexpr int csr_long_len(int lanes) { return kCsrLongGroups * csr_group(lanes) * lanes; }
+// Default lanes per row of a CSR matrix (tune.cu).
+int csr_lanes(const CsrDev &c, int32_t rows);
 template <class X>
 void spmv_csr_split(const CsrDev &c, int32_t m, const X *x, X *y, X alpha,
                     X beta, cudaStream_t s);
@@ -652,10 +661,10 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
                 cudaStream_t s);
 // First bad row (pointers decreasing or outside [0, nnz]) and first bad
 // entry (index outside [0, cols)) of 0-based compressed device arrays, -1
-// when none.
+// when none; the longest row (0 without rows) in *longest.
 std::pair<int64_t, int64_t> check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                              const int32_t *ptr, const int32_t *idx,
-                                             cudaStream_t s);
+                                             cudaStream_t s, int32_t *longest = nullptr);
 // COO (0-based device arrays, any order, duplicates allowed) -> CSR sorted by
 // (row, column), duplicates kept in input order. Returns -1, or the first
 // entry whose row or column is out of range (then `out` is untouched).

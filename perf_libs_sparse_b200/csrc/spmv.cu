@@ -30,36 +30,19 @@ __device__ __forceinline__ void store_y(X *y, int64_t i, Acc sum, X alpha,
 
 // ---------------------------------------------------------------- CSR
 
-// TPR lanes per row; rows longer than skip_len (when > 0) are left to the
-// long-row kernel.
-template <int TPR, class V, class X>
-__global__ void __launch_bounds__(256)
-    k_csr_vector(int32_t m, const int32_t *__restrict__ rp,
-                 const int32_t *__restrict__ col, const V *__restrict__ val,
-                 const X *__restrict__ x, X *__restrict__ y, X alpha, X beta,
-                 int beta_nz, int32_t skip_len) {
-  using Acc = typename AccOf<V, X>::type;
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t row = gid / TPR;
-  if (row >= m)
-    return;
-  const int sub = threadIdx.x & (TPR - 1);
-  const int32_t s = __ldg(rp + row), e = __ldg(rp + row + 1);
-  if (skip_len > 0 && e - s > skip_len)
-    return;  // uniform across the row's lanes
-  // Groups of G elements per lane: all value / column loads of a group are
-  // issued (predicated past the row end) before the dependent x gathers. One
-  // lane per row takes 8, so the short rows that configuration is picked for
-  // (stencils) cost one stream round trip and one gather round trip.
-  constexpr int G = TPR == 1 ? 8 : 4;
-  const L2Policy pol = make_l2_policy();
+// Sum over entries [j, e), `step` apart in the caller's lane: groups of G
+// elements per lane, all value / column loads of a group issued (predicated
+// past the end) before the dependent x gathers.
+template <int G, int STEP, class Acc, class V, class X>
+__device__ __forceinline__ Acc csr_lane_sum(uint32_t j, uint32_t e, const int32_t *col,
+                                            const V *val, const X *x, const L2Policy &pol) {
   Acc sum = 0;
-  for (int32_t j = s + sub; j < e; j += G * TPR) {
+  for (; j < e; j += G * STEP) {
     V v[G];
     int32_t c[G];
 #pragma unroll
     for (int u = 0; u < G; ++u) {
-      const int32_t q = j + u * TPR;
+      const uint32_t q = j + u * STEP;
       if (q < e) {
         v[u] = ld_stream(val + q, pol.stream);
         c[u] = ld_stream(col + q, pol.stream);
@@ -71,15 +54,64 @@ __global__ void __launch_bounds__(256)
     Acc xv[G];
 #pragma unroll
     for (int u = 0; u < G; ++u)
-      xv[u] = j + u * TPR < e ? to_acc<Acc>(ld_keep(x + c[u], pol.keep)) : Acc(0);
+      xv[u] = j + u * STEP < e ? to_acc<Acc>(ld_keep(x + c[u], pol.keep)) : Acc(0);
 #pragma unroll
     for (int u = 0; u < G; ++u)
-      if (j + u * TPR < e)
+      if (j + u * STEP < e)
         sum = fma(to_acc<Acc>(v[u]), xv[u], sum);
   }
+  return sum;
+}
+
+// TPR lanes per row; rows longer than skip_len (when > 0) are left to the
+// long-row kernel. One lane per row takes groups of 8, so the short rows that
+// configuration is picked for (stencils) cost one stream round trip and one
+// gather round trip. LONG: a row of more than kCsrLongGroups groups would keep
+// its TPR lanes, and with them the warp, in a long chain of round trips while
+// the warp's other lanes wait, so the whole warp takes such rows, one after
+// another (power-law rows of mean 16, 1 M of them: 182 us with the best lane
+// count, 117 us with this). The code for it takes the kernel from 32 to 40
+// registers, 5% on regular rows, so a matrix whose longest row needs it not
+// runs without.
+
+template <int TPR, bool LONG, class V, class X>
+__global__ void __launch_bounds__(256)
+    k_csr_vector(int32_t m, const int32_t *__restrict__ rp,
+                 const int32_t *__restrict__ col, const V *__restrict__ val,
+                 const X *__restrict__ x, X *__restrict__ y, X alpha, X beta,
+                 int beta_nz, int32_t skip_len) {
+  using Acc = typename AccOf<V, X>::type;
+  constexpr int G = csr_group(TPR);
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t row = gid / TPR;
+  const int sub = threadIdx.x & (TPR - 1);
+  bool live = row < m;
+  int32_t s = 0, e = 0;
+  if (live) {
+    s = __ldg(rp + row);
+    e = __ldg(rp + row + 1);
+    live = !(skip_len > 0 && e - s > skip_len);  // uniform across the row's lanes
+  }
+  const L2Policy pol = make_l2_policy();
+  const bool big = LONG && live && e - s > csr_long_len(TPR);
+  Acc sum = 0;
+  if (live && !big)
+    sum = csr_lane_sum<G, TPR, Acc>(s + sub, e, col, val, x, pol);
   if constexpr (TPR > 1)
-    sum = group_sum<TPR>(sum, group_mask<TPR>());
-  if (sub == 0)
+    sum = group_sum<TPR>(sum, 0xffffffffu);
+  if constexpr (LONG) {
+    unsigned todo = __ballot_sync(0xffffffffu, big && sub == 0);
+    while (todo) {
+      const int o = __ffs(todo) - 1;  // the row's first lane
+      todo &= todo - 1;
+      const int32_t s0 = __shfl_sync(0xffffffffu, s, o), e0 = __shfl_sync(0xffffffffu, e, o);
+      const Acc t = group_sum<32>(
+          csr_lane_sum<4, 32, Acc>(s0 + (threadIdx.x & 31), e0, col, val, x, pol), 0xffffffffu);
+      if ((threadIdx.x & 31) == o)
+        sum = t;
+    }
+  }
+  if (sub == 0 && live)
     store_y(y, row, sum, alpha, beta, beta_nz);
 }
 
@@ -117,7 +149,13 @@ static void launch_csr_vector(const CsrDev &c, int64_t r0, int32_t m, const X *x
                               X alpha, X beta, int32_t skip, cudaStream_t s) {
   const int64_t threads = (int64_t)m * TPR;
   const int64_t blocks = div_up(threads, 256);
-  k_csr_vector<TPR, V, X><<<(unsigned)blocks, 256, 0, s>>>(
+  // The long-row kernel beside this one (skip) takes the long rows itself.
+  const bool has_long = skip == 0 && c.max_row > csr_long_len(TPR);
+  auto kern = k_csr_vector<TPR, false, V, X>;
+  if constexpr (TPR < 32)
+    if (has_long)
+      kern = k_csr_vector<TPR, true, V, X>;
+  kern<<<(unsigned)blocks, 256, 0, s>>>(
       m, c.row_ptr.as<int32_t>() + r0, c.col.as<int32_t>(), (const V *)c.ev(), x, y + r0,
       alpha, beta, beta != X(0), skip);
 }

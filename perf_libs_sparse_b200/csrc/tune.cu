@@ -61,9 +61,31 @@ int64_t matrix_bytes(const Mat *A) {
 SpmvConfig default_config(const Mat *A) {
   SpmvConfig c;
   c.kind = Kind::CSR_VECTOR;
-  const double mean = A->m > 0 ? (double)A->csr.nnz / A->m : 1.0;
-  c.tpr = pow2_floor(mean);
+  c.tpr = csr_lanes(A->csr, A->m);
   return c;
+}
+
+// Each lane has a group of 4 entries in flight: as many lanes as cover the
+// longest row in one round trip, but no more than two for every three entries
+// of the mean row, since lanes past a row's end are idle slots, and at most 16
+// (a warp per row from a mean of 256). Where rows are long enough for the
+// whole-warp part (kCsrLongGroups), the lanes are for the short rows that most
+// rows of such a matrix are, and a quarter of the mean is the better size.
+// Measured (us; the power of two below the mean -> this rule): 5-point
+// Laplacian 2000^2 123 (4) -> 69 (2; 1 lane: 76), 27-point stencil 110^3
+// 145 (16) -> 85 (8; 4: 88), random 500,009 x 17 64 (16) -> 47 (8; 4: 53),
+// 100,009 x 32 27 (32) -> 21 (16; 8: 22), 311,479 FP32 rows of 12 on average
+// and up to 30 entries 22.8 (8) -> 22.8 (4: 23.8), bands of 129 118 (32) -> 87
+// (16); power-law rows of mean 16: 1 M 182 (16) -> 120 (4; 8: 137), 30,000
+// 50 (16) -> 34.
+int csr_lanes(const CsrDev &c, int32_t rows) {
+  const double mean = rows > 0 ? (double)c.nnz / rows : 1.0;
+  if (mean >= 256)
+    return 32;
+  int t = 1;
+  while (t < 16 && 4 * t < c.max_row && 2 * t <= mean / 1.5)
+    t *= 2;
+  return c.max_row > csr_long_len(t) ? std::min(16, pow2_floor(mean / 4)) : t;
 }
 
 // Make cfg the active SpMV configuration: build the SELL layout or the

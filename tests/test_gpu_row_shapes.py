@@ -50,3 +50,55 @@ def test_sell_slices_of_power_law_rows(rows, C_, sigma):
     scale = 1.25 * oracle.csr_absdot(rp, c, v, x) + 0.5 * np.abs(y0)
     for _ in range(2):  # the counts of the slices return to zero
         check(A.spmv(x, y0.copy(), alpha=1.25, beta=-0.5), ref, scale, 1e-12)
+
+
+# -------------------------------------------------------------------- CSR
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16, 32])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_csr_rows_around_the_whole_warp_length(lanes, dtype):
+    """Rows just below, at and above 4 groups of a row's lanes, in every
+    position of a warp, beside empty rows, and a last row alone in its warp."""
+    rng = np.random.default_rng(lanes)
+    t = 4 * (8 if lanes == 1 else 4) * lanes
+    n = 6000
+    lens = [0, 1, t - 1, t, t + 1, 2 * t + 3, 0, 5000, 3, t + 1, t + 2] + [2] * 70
+    lens += list(rng.integers(0, t + 2, 61)) + [t + 5]
+    rp, c, v = csr_of_lengths(lens, n, rng)
+    m = len(lens)
+    v = v.astype(dtype)
+    x, y0 = W.uniform_vector(n, 4).astype(dtype), W.uniform_vector(m, 5).astype(dtype)
+    A = pls.SpMat.csr(m, n, rp, c, v)
+    assert A.force_config(pls.KIND_CSR, 0, 0, lanes) == 0
+    assert A.optimize() == 0
+    for alpha, beta in ((1.0, 0.0), (1.5, -0.25)):
+        ref = oracle.csr_spmv(rp, c, v.astype(np.float64), x.astype(np.float64),
+                              y=y0.astype(np.float64), alpha=alpha, beta=beta)
+        scale = alpha * oracle.csr_absdot(rp, c, v.astype(np.float64), x.astype(np.float64)) \
+            + abs(beta) * np.abs(y0.astype(np.float64))
+        y = A.spmv(x, np.full(m, np.nan, dtype) if beta == 0 else y0.copy(), alpha=alpha, beta=beta)
+        check(y, ref, scale, 1e-12 if dtype == np.float64 else 1e-5)
+
+
+def test_csr_default_lanes_on_every_creation_path():
+    """The default kernel where the longest row is known from the arrays the
+    library made itself: COO, CSC and the transposed operation."""
+    rng = np.random.default_rng(7)
+    n = 900
+    rp, c, v = csr_of_lengths([3] * 500 + [700] + [5] * 399, n, rng)
+    m = len(rp) - 1
+    x = W.uniform_vector(n, 8)
+    ref, scale = oracle.csr_spmv(rp, c, v, x), oracle.csr_absdot(rp, c, v, x)
+    rows = np.repeat(np.arange(m, dtype=np.int32), np.diff(rp))
+    check(pls.SpMat.coo(m, n, rows, c, v).spmv(x), ref, scale, 1e-12)
+    order = np.lexsort((rows, c))
+    cp = np.zeros(n + 1, np.int32)
+    cp[1:] = np.cumsum(np.bincount(c, minlength=n))
+    check(pls.SpMat.csc(m, n, rows[order], cp, v[order]).spmv(x), ref, scale, 1e-12)
+    A = pls.SpMat.csr(m, n, rp, c, v)
+    A.hint(pls.HINT_SPMV_OPERATION, pls.OPERATION_TRANS)
+    assert A.optimize() == 0
+    xt = W.uniform_vector(m, 9)
+    check(A.spmv(xt, trans=pls.OPERATION_TRANS), oracle.csr_spmv_trans(rp, c, v, n, xt),
+          oracle.csr_spmv_trans(rp, c, np.abs(v), n, np.abs(xt)), 1e-12)

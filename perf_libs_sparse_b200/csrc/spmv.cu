@@ -10,7 +10,9 @@
 //   * grids launch one thread group per row / chunk and let the block
 //     scheduler balance uneven rows across the 148 SMs.
 #include <algorithm>
+#include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "pls_internal.hpp"
@@ -841,42 +843,110 @@ void spmv_dense(const DenseDev &d, int32_t m, int32_t n, bool trans,
 
 // ---------------------------------------------------------------- BSR
 
-// Block sizes whose bs*bs elements tile a warp (bs = 1, 2, 4): a warp per
-// block row; lane l owns element e = l % (bs*bs) of 32/(bs*bs) consecutive
-// blocks per step, so every step reads 32 consecutive values. Lanes holding
-// the same scalar row are reduced with shuffles at the end.
-template <int BS, class V, class X>
-__global__ void __launch_bounds__(256)
-    k_bsr_small(int32_t mb, int layout, const int32_t *__restrict__ rp,
-                const int32_t *__restrict__ col, const V *__restrict__ val,
-                const X *__restrict__ x, X *__restrict__ y, X alpha, X beta,
-                int beta_nz) {
-  using Acc = typename AccOf<V, X>::type;
-  constexpr int E = BS * BS, PER = 32 / E;
-  const int64_t br = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  if (br >= mb)
-    return;
-  const int lane = threadIdx.x & 31, e = lane % E, slot = lane / E;
-  const bool rm = layout == PERFLIBS_ROW_MAJOR;
-  const int i = rm ? e / BS : e % BS;
-  const int j = rm ? e % BS : e / BS;
-  Acc acc = 0;
-  for (int32_t b = rp[br] + slot; b < rp[br + 1]; b += PER) {
-    const Acc v = to_acc<Acc>(ld_stream(val + (int64_t)b * E + e));
-    acc = fma(v, to_acc<Acc>(ld_ro(x + (int64_t)ld_stream(col + b) * BS + j)), acc);
+// K consecutive values at p: whole 16-byte vectors (8 or 4 bytes when K
+// elements are fewer) with VECT (p is then aligned to them), else one by one;
+// STREAM marks whole vectors read once.
+template <int K, bool VECT, bool STREAM, class T>
+__device__ __forceinline__ void ld_consecutive(const T *p, T (&v)[K]) {
+  constexpr int bytes = K * (int)sizeof(T);
+  if constexpr (!VECT || bytes < 4 || K == 1) {
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      v[i] = __ldg(p + i);
+  } else if constexpr (bytes == 4) {
+    const unsigned t = __ldg(reinterpret_cast<const unsigned *>(p));
+    memcpy(v, &t, 4);
+  } else if constexpr (bytes == 8) {
+    const uint2 t = __ldg(reinterpret_cast<const uint2 *>(p));
+    memcpy(v, &t, 8);
+  } else {
+    static_assert(bytes % 16 == 0, "whole vectors");
+#pragma unroll
+    for (int h = 0; h < bytes / 16; ++h) {
+      const uint4 t = STREAM ? __ldcs(reinterpret_cast<const uint4 *>(p) + h)
+                             : __ldg(reinterpret_cast<const uint4 *>(p) + h);
+      memcpy(reinterpret_cast<char *>(v) + 16 * h, &t, 16);
+    }
   }
-  // Reduce over all lanes with the same i: the j bits and the slot bits.
+}
+
+// Block sizes 1, 2, 4, 8: G = 2^lg_g lanes per block row. A lane owns W
+// consecutive values of every block it takes (one 16-byte load; fewer for
+// blocks below 16 bytes), LPB lanes a whole block, so the G / LPB lane sets of
+// a block row read consecutive blocks and a warp load covers consecutive
+// memory. The lane's values lie on NR rows and NC columns of the block: it
+// loads the NC elements of x once per block and keeps NR partial sums, added
+// over the lanes of the block row at the end.
+//
+// Bound by HBM latency and bandwidth: the values are read once and x mostly
+// from L2. One block per lane set and step, its column loaded a step ahead,
+// keeps the kernel near 32 registers, and full occupancy hides more latency
+// than loads in flight per lane do (2 blocks in flight: 49 against 45 us, 4:
+// 63 us, on the first matrix below). Measured (FP64, warm; a thread per scalar
+// row for bs = 8, a warp per block row and one value per lane for bs 2 and 4
+// -> this kernel): bs 8, 60,011 x 8 random blocks 83.6 -> 45.3 us (39 us at
+// the copy rate), bs 4, 100,000 x 6 24.8 -> 19.4 us, bs 2, 300,000 x 12
+// 61.8 -> 28.9 us; bs 8 with BF16 values and FP32 x 41.2 -> 16.7 us.
+template <int BS, bool RM, bool XVEC, class V, class X>
+__global__ void __launch_bounds__(256)
+    k_bsr_vec(int32_t mb, int lg_g, const int32_t *__restrict__ rp,
+              const int32_t *__restrict__ col, const V *__restrict__ val,
+              const X *__restrict__ x, X *__restrict__ y, X alpha, X beta, int beta_nz) {
+  using Acc = typename AccOf<V, X>::type;
+  constexpr int E = BS * BS;
+  constexpr int WV = 16 / (int)sizeof(V);
+  constexpr int W = WV < E ? WV : E;    // values per lane and block
+  constexpr int LPB = E / W;            // lanes per block
+  constexpr int RUN = W < BS ? W : BS;  // consecutive values on one block line
+  constexpr int LINES = W / RUN;        // block lines (rows when RM) per lane
+  constexpr int NR = RM ? LINES : RUN, NC = RM ? RUN : LINES;
+  const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int64_t br = t >> lg_g;
+  const int G = 1 << lg_g;
+  const int g = (int)threadIdx.x & (G - 1);
+  const int e0 = (g % LPB) * W;  // the lane's first value in a block
+  const int line = e0 / BS, at = e0 % BS;
+  const int i0 = RM ? line : at, j0 = RM ? at : line;
+  const uint32_t step = G / LPB;
+  uint32_t b = 0, b1 = 0;  // unsigned: b + step passes 2^31 without overflow
+  if (br < mb) {
+    b = (uint32_t)__ldg(rp + br) + g / LPB;
+    b1 = (uint32_t)__ldg(rp + br + 1);
+  }
+  Acc acc[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+    acc[r] = Acc(0);
+  int32_t next = b < b1 ? __ldg(col + b) : 0;
+  while (b < b1) {
+    const int32_t c = next;
+    V a[W];
+    ld_consecutive<W, true, true>(val + (int64_t)b * E + e0, a);
+    X xv[NC];
+    ld_consecutive<NC, XVEC, false>(x + (int64_t)c * BS + j0, xv);
+    b += step;
+    next = b < b1 ? __ldg(col + b) : 0;
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int j = 0; j < NC; ++j)
+        acc[r] = fma(to_acc<Acc>(a[RM ? r * RUN + j : j * RUN + r]), to_acc<Acc>(xv[j]), acc[r]);
+  }
+  // Add over the lanes that hold the same rows: those of the block's other
+  // columns and of the other lane sets.
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int lo = rm ? o : o;  // lane bit o
-    const bool is_i_bit = rm ? (o >= BS && o < E) : (o < BS);
-    if (!is_i_bit)
-      acc += __shfl_xor_sync(0xffffffffu, acc, lo);
+    const bool rows_differ = o < LPB && (RM ? o * W >= BS : o * W < BS);
+    if (!rows_differ && o < G) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+    }
   }
-  const bool owner = rm ? (j == 0 && slot == 0) : (j == 0 && slot == 0);
-  if (owner) {
-    const int64_t r = br * BS + i;
-    store_y(y, r, acc, alpha, beta, beta_nz);
+  if (br < mb && g < LPB && j0 == 0) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      store_y(y, br * BS + i0 + r, acc[r], alpha, beta, beta_nz);
   }
 }
 
@@ -918,20 +988,39 @@ void spmv_bsr(const BsrDev &b, const X *x, X *y, X alpha, X beta,
     if constexpr (std::is_same_v<X, float> && std::is_same_v<V, double>) {
       throw Error(PERFLIBS_STATUS_EXECUTION_FAILURE, "FP64 storage with FP32 API");
     } else {
-      const unsigned wblocks = (unsigned)div_up((int64_t)b.mb * 32, 256);
+      const auto vec = [&](auto bs_tag, auto rm_tag) {
+        constexpr int BS = decltype(bs_tag)::value;
+        constexpr bool RM = decltype(rm_tag)::value;
+        constexpr int WV = 16 / (int)sizeof(V), W = WV < BS * BS ? WV : BS * BS;
+        // Lanes per block row: half as many block-wide lane sets as a block
+        // row has blocks (a power of two), up to a warp. As many sets as
+        // blocks leave each lane one block between its row pointer load and
+        // its reduction (bs 4, 6 blocks: 24.8 against 19.4 us; bs 2, 12
+        // blocks: 35.0 against 28.9 us); a quarter as many gain nothing more
+        // (18.6 and 29.3 us).
+        int lg_g = 0;
+        while ((1 << lg_g) < BS * BS / W)
+          ++lg_g;
+        const double mean = (double)b.nnzb / b.mb;
+        for (int sets = 2; 2 * sets <= mean && lg_g < 5; sets *= 2)
+          ++lg_g;
+        const unsigned grid = (unsigned)div_up((int64_t)b.mb << lg_g, 256);
+        const bool xvec = (uintptr_t)x % 16 == 0;  // else x is read element by element
+        auto kern = xvec ? k_bsr_vec<BS, RM, true, V, X> : k_bsr_vec<BS, RM, false, V, X>;
+        kern<<<grid, 256, 0, s>>>(b.mb, lg_g, b.row_ptr.as<int32_t>(), b.col.as<int32_t>(),
+                                  (const V *)b.ev(), x, y, alpha, beta, bnz);
+      };
+      const auto by_layout = [&](auto bs_tag) {
+        if (b.layout == PERFLIBS_ROW_MAJOR)
+          vec(bs_tag, std::true_type{});
+        else
+          vec(bs_tag, std::false_type{});
+      };
       switch (b.bs) {
-      case 1:
-        k_bsr_small<1, V, X><<<wblocks, 256, 0, s>>>(b.mb, b.layout, b.row_ptr.as<int32_t>(),
-            b.col.as<int32_t>(), (const V *)b.ev(), x, y, alpha, beta, bnz);
-        break;
-      case 2:
-        k_bsr_small<2, V, X><<<wblocks, 256, 0, s>>>(b.mb, b.layout, b.row_ptr.as<int32_t>(),
-            b.col.as<int32_t>(), (const V *)b.ev(), x, y, alpha, beta, bnz);
-        break;
-      case 4:
-        k_bsr_small<4, V, X><<<wblocks, 256, 0, s>>>(b.mb, b.layout, b.row_ptr.as<int32_t>(),
-            b.col.as<int32_t>(), (const V *)b.ev(), x, y, alpha, beta, bnz);
-        break;
+      case 1: by_layout(std::integral_constant<int, 1>{}); break;
+      case 2: by_layout(std::integral_constant<int, 2>{}); break;
+      case 4: by_layout(std::integral_constant<int, 4>{}); break;
+      case 8: by_layout(std::integral_constant<int, 8>{}); break;
       default:
         k_bsr_rows<V, X><<<(unsigned)div_up((int64_t)b.mb * b.bs, 256), 256, 0, s>>>(
             b.mb, b.bs, b.layout, b.row_ptr.as<int32_t>(), b.col.as<int32_t>(),

@@ -102,3 +102,42 @@ def test_csr_default_lanes_on_every_creation_path():
     xt = W.uniform_vector(m, 9)
     check(A.spmv(xt, trans=pls.OPERATION_TRANS), oracle.csr_spmv_trans(rp, c, v, n, xt),
           oracle.csr_spmv_trans(rp, c, np.abs(v), n, np.abs(xt)), 1e-12)
+
+
+# -------------------------------------------------------------------- BSR
+
+
+@pytest.mark.parametrize("bs", [1, 2, 4, 8])
+@pytest.mark.parametrize("layout", [pls.ROW_MAJOR, pls.COL_MAJOR])
+@pytest.mark.parametrize("dtype,storage", [(np.float64, "native"), (np.float64, "bf16"), (np.float64, "fp32"),
+                                           (np.float32, "native"), (np.float32, "bf16")])
+def test_bsr_spmv_block_shapes(bs, layout, dtype, storage):
+    """Block rows of 0 to 40 blocks, a number of block rows that fills no
+    warp, and x off a 16-byte boundary."""
+    import torch
+
+    rng = np.random.default_rng(bs)
+    for mb, per in ((37, 3), (5, 40), (1, 1), (130, 12)):
+        nb = 45
+        lens = rng.integers(0, per + 1, mb)
+        lens[0] = per
+        rp, c, _ = csr_of_lengths(lens, nb, rng)
+        # values that BF16 holds exactly
+        v = (rng.integers(-128, 129, int(rp[-1]) * bs * bs) / 64).astype(dtype)
+        m, n = mb * bs, nb * bs
+        A = pls.SpMat.bsr(layout, m, n, bs, rp, c, v)
+        A.set_storage({"native": pls.STORAGE_NATIVE, "fp32": pls.STORAGE_FP32,
+                       "bf16": pls.STORAGE_BF16}[storage])
+        x, y0 = W.uniform_vector(n + 1, 4).astype(dtype), W.uniform_vector(m, 5).astype(dtype)
+        xd = torch.tensor(x, device="cuda")
+        tol = 1e-12 if dtype == np.float64 and storage == "native" else 1e-5
+        for off in (0, 1):
+            xs = x[off:off + n].astype(np.float64)
+            v64 = v.astype(np.float64)
+            ref = oracle.bsr_spmv(rp, c, v64, bs, layout, xs, y=y0.astype(np.float64), alpha=0.5, beta=2.0)
+            scale = 0.5 * oracle.bsr_spmv(rp, c, np.abs(v64), bs, layout, np.abs(xs)) + 2 * np.abs(y0.astype(np.float64))
+            yd = torch.tensor(y0, device="cuda")
+            torch.cuda.synchronize()
+            A.spmv_dev(xd.data_ptr() + off * x.itemsize, yd.data_ptr(), 0.5, 2.0)
+            torch.cuda.synchronize()
+            check(yd.cpu().numpy(), ref, scale, tol)

@@ -784,6 +784,28 @@ int64_t count_blocks(const CsrDev &c, int32_t m, int32_t n, int bs, cudaStream_t
   return last;
 }
 
+void list_long_rows(const DevBuf &row_ptr, int32_t m, int threshold, DevBuf &rows,
+                    std::vector<int32_t> &lens, cudaStream_t s) {
+  std::vector<int32_t> rp((size_t)m + 1);
+  PLS_CUDA(cudaMemcpyAsync(rp.data(), row_ptr.p, sizeof(int32_t) * rp.size(),
+                           cudaMemcpyDeviceToHost, s));
+  PLS_CUDA(cudaStreamSynchronize(s));
+  std::vector<int32_t> list;
+  for (int32_t r = 0; r < m; ++r)
+    if (rp[r + 1] - rp[r] > threshold)
+      list.push_back(r);
+  std::stable_sort(list.begin(), list.end(), [&](int32_t a, int32_t b) {
+    return rp[a + 1] - rp[a] > rp[b + 1] - rp[b];
+  });
+  lens.clear();
+  for (const int32_t r : list)
+    lens.push_back(rp[r + 1] - rp[r]);
+  rows.reserve(sizeof(int32_t) * std::max<size_t>(list.size(), 1));
+  PLS_CUDA(cudaMemcpyAsync(rows.p, list.data(), sizeof(int32_t) * list.size(),
+                           cudaMemcpyHostToDevice, s));
+  PLS_CUDA(cudaStreamSynchronize(s));
+}
+
 void csr_build_long_rows(CsrDev &c, int32_t m, int threshold, cudaStream_t s) {
   c.bands.clear();
   c.long_threshold = threshold;

@@ -392,6 +392,11 @@ struct CsrDev {
   DevBuf long_rows;
   int n_long = 0;
   int long_threshold = 0;
+  // Rows far longer than the mean, longest first, with their lengths: the
+  // SpMM gives them whole CTAs (found on the first SpMM).
+  bool wide_found = false;
+  DevBuf wide_rows;
+  std::vector<int32_t> wide_len;
   // Staged-SpMM tiles (built on the first suitable SpMM).
   TileDev tiles;
   DiaDev dia;
@@ -672,6 +677,9 @@ int64_t coo_to_csr(int32_t m, int32_t n, int64_t nnz, const int32_t *row, const 
                    const void *vals, Vt vt, CsrDev &out, cudaStream_t s);
 void csr_to_bsr(const CsrDev &c, int32_t m, int32_t n, int bs, int layout,
                 BsrDev &out, cudaStream_t s);
+// Rows of more than `threshold` entries, longest first, and their lengths.
+void list_long_rows(const DevBuf &row_ptr, int32_t m, int threshold, DevBuf &rows,
+                    std::vector<int32_t> &lens, cudaStream_t s);
 void csr_build_long_rows(CsrDev &c, int32_t m, int threshold, cudaStream_t s);
 
 // Norms (double accumulate on device, result to host).

@@ -10,6 +10,8 @@
 //
 // BSR: a warp per block row, lanes over C's columns; each lane keeps bs
 // accumulators (one per scalar row of the block row).
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -19,8 +21,16 @@
 
 namespace pls {
 
-template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES>
-__device__ __forceinline__ void spmm_csr_rows(int32_t m, int lg_tk, int lg_tn,
+// What a row-group launch computes beside the row groups: the n wide rows
+// (longer than `skip`, listed longest first), `tiles` column tiles each, take
+// the first n * tiles CTAs.
+struct WideRows {
+  const int32_t *rows;
+  int32_t n, skip, tiles;
+};
+
+template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES, bool WIDE>
+__device__ __forceinline__ void spmm_csr_rows(int32_t m, int lg_tk, int lg_tn, const WideRows &w,
                                               const int32_t *__restrict__ rp,
                                               const int32_t *__restrict__ col,
                                               const V *__restrict__ val, const X *__restrict__ B,
@@ -28,22 +38,35 @@ __device__ __forceinline__ void spmm_csr_rows(int32_t m, int lg_tk, int lg_tn,
                                               X alpha, X beta, int beta_nz) {
   using Acc = typename AccOf<V, X>::type;
   const L2Policy pol = make_l2_policy();
+  const CsrRows<V, WIDE> A{rp, col, val, w.skip};
+  int64_t block = blockIdx.x;
+  if constexpr (WIDE) {
+    __shared__ Acc part[256 * VEC];
+    const int64_t wide = (int64_t)w.n * w.tiles;
+    if (block < wide) {
+      const int32_t row = __ldg(w.rows + block / w.tiles);
+      spmm_wide_row<VEC, Acc, X, CsrRows<V, WIDE>, OFF32>(
+          A, __ldg(rp + row), __ldg(rp + row + 1), row, (int)(block % w.tiles), lg_tk, B, ldb, C,
+          ldc, k, alpha, beta, beta_nz, part, pol);
+      return;
+    }
+    block -= wide;
+  }
   const int lg_g = lg_tk + lg_tn;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
   const int64_t row = (warp << (5 - lg_g)) + ((threadIdx.x & 31) >> lg_g);
-  const CsrRows<V> A{rp, col, val};
-  spmm_row_group<VEC, NV, Acc, X, CsrRows<V>, OFF32, ENTRIES>(
+  spmm_row_group<VEC, NV, Acc, X, CsrRows<V, WIDE>, OFF32, ENTRIES>(
       A, row, row < m, lg_tk, lg_tn, B, ldb, C, ldc, k, alpha, beta, beta_nz, pol);
 }
 
-template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES>
+template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES, bool WIDE>
 __global__ void __launch_bounds__(256)
-    k_spmm_csr(int32_t m, int lg_tk, int lg_tn, const int32_t *__restrict__ rp,
+    k_spmm_csr(int32_t m, int lg_tk, int lg_tn, WideRows w, const int32_t *__restrict__ rp,
                const int32_t *__restrict__ col, const V *__restrict__ val,
                const X *__restrict__ B, int64_t ldb, X *__restrict__ C, int64_t ldc, int k,
                X alpha, X beta, int beta_nz) {
-  spmm_csr_rows<VEC, NV, V, X, OFF32, ENTRIES>(m, lg_tk, lg_tn, rp, col, val, B, ldb, C, ldc, k,
-                                               alpha, beta, beta_nz);
+  spmm_csr_rows<VEC, NV, V, X, OFF32, ENTRIES, WIDE>(m, lg_tk, lg_tn, w, rp, col, val, B, ldb, C,
+                                                     ldc, k, alpha, beta, beta_nz);
 }
 
 // Shared entries for FP32 results with one vector per lane, held to 48
@@ -53,14 +76,14 @@ __global__ void __launch_bounds__(256)
 // k = 32 0.598 / 0.628 / 0.591 ms, k = 128 2.141 / 2.180 / 2.019 ms. FP64
 // results spill at the cap and run uncapped (k = 8 0.494 / 0.388 / 0.505,
 // k = 32 1.39 / 1.18 / 1.26), as do two vectors per lane (NV = 2).
-template <int VEC, class V, class X, bool OFF32>
+template <int VEC, class V, class X, bool OFF32, bool WIDE>
 __global__ void __launch_bounds__(256, 5)
-    k_spmm_csr_shared(int32_t m, int lg_tk, int lg_tn, const int32_t *__restrict__ rp,
-                      const int32_t *__restrict__ col, const V *__restrict__ val,
-                      const X *__restrict__ B, int64_t ldb, X *__restrict__ C, int64_t ldc,
-                      int k, X alpha, X beta, int beta_nz) {
-  spmm_csr_rows<VEC, 1, V, X, OFF32, kEntriesShared>(m, lg_tk, lg_tn, rp, col, val, B, ldb, C,
-                                                     ldc, k, alpha, beta, beta_nz);
+    k_spmm_csr_shared(int32_t m, int lg_tk, int lg_tn, WideRows w,
+                      const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
+                      const V *__restrict__ val, const X *__restrict__ B, int64_t ldb,
+                      X *__restrict__ C, int64_t ldc, int k, X alpha, X beta, int beta_nz) {
+  spmm_csr_rows<VEC, 1, V, X, OFF32, kEntriesShared, WIDE>(m, lg_tk, lg_tn, w, rp, col, val, B,
+                                                           ldb, C, ldc, k, alpha, beta, beta_nz);
 }
 
 // 32-bit address arithmetic is possible when every offset into B (rows
@@ -68,6 +91,29 @@ __global__ void __launch_bounds__(256, 5)
 // column count was not recorded.
 static bool rows_off32_fits(const CsrDev &c, int32_t m, int64_t ldb, int64_t ldc) {
   return c.ncols > 0 && (int64_t)c.ncols * ldb < INT32_MAX && (int64_t)m * ldc < INT32_MAX;
+}
+
+// Lists the rows far longer than the mean (more than 8 times it, and 128
+// entries), longest first, on the first SpMM of a matrix that has any. Under
+// stream capture nothing is built and they run as any other row.
+constexpr int kWideRow = 128;
+constexpr int kWideMean = 8;
+
+static void find_wide_rows(CsrDev &c, int32_t m, cudaStream_t s) {
+  if (c.wide_found || m <= 0)
+    return;
+  const int32_t thr =
+      (int32_t)std::max<double>(kWideRow, kWideMean * std::ceil((double)c.nnz / m));
+  if (c.max_row <= thr) {
+    c.wide_found = true;
+    return;
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  PLS_CUDA(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone)
+    return;
+  list_long_rows(c.row_ptr, m, thr, c.wide_rows, c.wide_len, s);
+  c.wide_found = true;
 }
 
 // Whether the shared-entries mode applies to this lane shape: one lane group
@@ -81,7 +127,18 @@ static bool launch_spmm_csr(const CsrDev &c, int32_t m, const X *B, int64_t ldb,
                             cudaStream_t s) {
   const RowsShape sh = rows_shape(k, VEC, (double)c.nnz / std::max<int32_t>(m, 1));
   const int64_t rows_per_block = (int64_t)8 << (5 - (sh.lg_tk + sh.lg_tn));
-  const unsigned blocks = (unsigned)div_up(m, rows_per_block);
+  // Wide rows: those with entries for every group of a CTA; shorter ones
+  // would leave part of it idle.
+  WideRows w{nullptr, 0, INT32_MAX, 1};
+  if (!c.wide_len.empty()) {
+    w.rows = c.wide_rows.as<int32_t>();
+    w.skip = std::max(c.wide_len.back() - 1, kSpmmInFlight * (256 >> sh.lg_tk));
+    w.n = (int32_t)(std::partition_point(c.wide_len.begin(), c.wide_len.end(),
+                                         [&](int32_t l) { return l > w.skip; }) -
+                    c.wide_len.begin());
+    w.tiles = (int32_t)div_up(k, (int64_t)VEC << sh.lg_tk);
+  }
+  const unsigned blocks = (unsigned)(div_up(m, rows_per_block) + (int64_t)w.n * w.tiles);
   const int bnz = beta != X(0);
   off32 = off32 && rows_off32_fits(c, m, ldb, ldc);
   shared = shared && shared_entries_fit(sh);
@@ -89,14 +146,15 @@ static bool launch_spmm_csr(const CsrDev &c, int32_t m, const X *B, int64_t ldb,
     constexpr int NV = decltype(nv_tag)::value;
     constexpr bool OFF = decltype(off_tag)::value;
     constexpr int EM = decltype(entries_tag)::value;
+    auto kern = k_spmm_csr<VEC, NV, V, X, OFF, EM, false>;
     if constexpr (EM == kEntriesShared && NV == 1 && sizeof(X) == 4)
-      k_spmm_csr_shared<VEC, V, X, OFF><<<blocks, 256, 0, s>>>(m, sh.lg_tk, sh.lg_tn,
-          c.row_ptr.as<int32_t>(), c.col.as<int32_t>(), (const V *)c.ev(), B, ldb, C, ldc, k,
-          alpha, beta, bnz);
-    else
-      k_spmm_csr<VEC, NV, V, X, OFF, EM><<<blocks, 256, 0, s>>>(m, sh.lg_tk, sh.lg_tn,
-          c.row_ptr.as<int32_t>(), c.col.as<int32_t>(), (const V *)c.ev(), B, ldb, C, ldc, k,
-          alpha, beta, bnz);
+      kern = w.n > 0 ? k_spmm_csr_shared<VEC, V, X, OFF, true>
+                     : k_spmm_csr_shared<VEC, V, X, OFF, false>;
+    else if (w.n > 0)
+      kern = k_spmm_csr<VEC, NV, V, X, OFF, EM, true>;
+    kern<<<blocks, 256, 0, s>>>(m, sh.lg_tk, sh.lg_tn, w, c.row_ptr.as<int32_t>(),
+                                c.col.as<int32_t>(), (const V *)c.ev(), B, ldb, C, ldc, k, alpha,
+                                beta, bnz);
   };
   using I1 = std::integral_constant<int, 1>;
   using I2 = std::integral_constant<int, 2>;
@@ -137,8 +195,9 @@ static int rows_vec(const CsrDev &c, int32_t m, const X *B, int64_t ldb, const X
 // arithmetic when `off32` and the offsets fit, and shared entry loads when
 // `shared` and the lane shape allows them (returns whether they ran).
 template <class X>
-static bool spmm_rows(const CsrDev &c, int32_t m, const X *B, int64_t ldb, X *C, int64_t ldc,
+static bool spmm_rows(CsrDev &c, int32_t m, const X *B, int64_t ldb, X *C, int64_t ldc,
                       int k, X alpha, X beta, bool off32, bool shared, cudaStream_t s) {
+  find_wide_rows(c, m, s);
   const int vec = rows_vec<X>(c, m, B, ldb, C, ldc, k, shared);
   bool ran = false;
   with_vt(c.evt(), [&](auto tag) {

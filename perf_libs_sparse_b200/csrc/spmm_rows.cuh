@@ -75,17 +75,25 @@ __device__ __forceinline__ void st_vec(X *p, const X (&v)[VEC]) {
 }
 
 // ---- rows of A as the loop reads them -----------------------------------
-// range(row) gives the row's entry interval [s, e) and an auxiliary word;
-// entry(q, aux) gives entry q's column of B and its value.
+// range(row) gives the row's entry interval [s, e) and an auxiliary word, and
+// says whether the loop computes the row; entry(q, aux) gives entry q's column
+// of B and its value.
 
-template <class Val> struct CsrRows {
+// With WIDE, rows of more than `skip` entries are left to whole CTAs.
+template <class Val, bool WIDE = false> struct CsrRows {
   using V = Val;
   const int32_t *rp, *col;
   const V *val;
-  __device__ __forceinline__ void range(int64_t r, int32_t &s, int32_t &e, int32_t &aux) const {
+  int32_t skip;
+  __device__ __forceinline__ bool range(int64_t r, int32_t &s, int32_t &e, int32_t &aux) const {
     s = __ldg(rp + r);
     e = __ldg(rp + r + 1);
     aux = 0;
+    if (WIDE && e - s > skip) {
+      e = s;
+      return false;
+    }
+    return true;
   }
   __device__ __forceinline__ void entry(int32_t q, int32_t, int32_t &c, V &a,
                                         const L2Policy &pol) const {
@@ -100,10 +108,11 @@ struct PackedRows {
   using V = float;
   const int32_t *rp;
   const int2 *cv;
-  __device__ __forceinline__ void range(int64_t r, int32_t &s, int32_t &e, int32_t &aux) const {
+  __device__ __forceinline__ bool range(int64_t r, int32_t &s, int32_t &e, int32_t &aux) const {
     s = __ldg(rp + r);
     e = __ldg(rp + r + 1);
     aux = 0;
+    return true;
   }
   __device__ __forceinline__ void entry(int32_t q, int32_t, int32_t &c, float &a,
                                         const L2Policy &pol) const {
@@ -151,7 +160,7 @@ __device__ __forceinline__ void spmm_row_group(const Rows &A, int64_t row, bool 
   const int tn = (lane >> lg_tk) & (TN - 1);
   int32_t s = 0, e = 0, aux = 0;
   if (live)
-    A.range(row, s, e, aux);
+    live = A.range(row, s, e, aux);
   int32_t longest = 0;  // kEntriesShared: the warp's longest row
   if constexpr (ENTRIES == kEntriesShared) {
     longest = e - s;
@@ -292,6 +301,84 @@ __device__ __forceinline__ void spmm_row_group(const Rows &A, int64_t row, bool 
         }
       }
     }
+  }
+}
+
+// A row far longer than the others, by a whole 256-thread CTA: 2^lg_tk lanes
+// of one vector over a tile of C's columns (tile t starts at column
+// t * TK * VEC), 256 / TK groups over the row's entries, U entries in flight
+// per lane; the groups' sums are added in a tree through shared memory
+// (256 * VEC elements at `part`). In the row-group loop such a row is a chain
+// of len / U round trips that the launch waits for.
+template <int VEC, class Acc, class X, class Rows, bool OFF32>
+__device__ __forceinline__ void spmm_wide_row(const Rows &A, int32_t s, int32_t e, int64_t row,
+                                              int tile, int lg_tk, const X *__restrict__ B,
+                                              int64_t ldb, X *__restrict__ C, int64_t ldc, int k,
+                                              X alpha, X beta, int beta_nz, Acc *part,
+                                              const L2Policy &pol) {
+  constexpr int U = kSpmmInFlight;
+  const int TK = 1 << lg_tk, groups = 256 >> lg_tk;
+  const int tk = (int)threadIdx.x & (TK - 1), g = (int)threadIdx.x >> lg_tk;
+  const int kk = (tile * TK + tk) * VEC;
+  Acc acc[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v)
+    acc[v] = Acc(0);
+  for (uint32_t p = (uint32_t)s + g; p < (uint32_t)e; p += U * groups) {
+    int32_t c[U];
+    Acc a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t q = p + u * groups;
+      if (q < (uint32_t)e) {
+        typename Rows::V av;
+        A.entry((int32_t)q, 0, c[u], av, pol);
+        a[u] = to_acc<Acc>(av);
+      } else {
+        c[u] = -1;
+        a[u] = Acc(0);
+      }
+    }
+    X b[U][VEC];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int32_t cu = c[u] < 0 ? 0 : c[u];
+      const X *bp = OFF32 ? B + (cu * (int32_t)ldb + kk) : B + (int64_t)cu * ldb + kk;
+      if (c[u] >= 0 && kk + VEC <= k) {
+        ld_vec<X, VEC>(bp, b[u]);
+      } else {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+          b[u][v] = (c[u] >= 0 && kk + v < k) ? __ldg(bp + v) : X(0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int v = 0; v < VEC; ++v)
+        acc[v] = fma(a[u], to_acc<Acc>(b[u][v]), acc[v]);
+  }
+  Acc *mine = part + threadIdx.x * VEC;
+#pragma unroll
+  for (int v = 0; v < VEC; ++v)
+    mine[v] = acc[v];
+  for (int o = groups / 2; o > 0; o >>= 1) {
+    __syncthreads();
+    if (g < o)
+#pragma unroll
+      for (int v = 0; v < VEC; ++v)
+        mine[v] += mine[o * TK * VEC + v];
+  }
+  if (g == 0) {
+    X *crow = C + row * ldc;
+#pragma unroll
+    for (int v = 0; v < VEC; ++v)
+      if (kk + v < k) {
+        X o = (X)mine[v] * alpha;
+        if (beta_nz)
+          o += beta * crow[kk + v];
+        crow[kk + v] = o;
+      }
   }
 }
 

@@ -141,3 +141,74 @@ def test_bsr_spmv_block_shapes(bs, layout, dtype, storage):
             A.spmv_dev(xd.data_ptr() + off * x.itemsize, yd.data_ptr(), 0.5, 2.0)
             torch.cuda.synchronize()
             check(yd.cpu().numpy(), ref, scale, tol)
+
+
+# ---------------------------------------------------------- SpMM, wide rows
+
+
+@pytest.mark.parametrize("k", [1, 6, 8, 33, 64, 130, 264])
+@pytest.mark.parametrize("dtype,storage", [(np.float64, "native"), (np.float32, "native"), (np.float32, "bf16")])
+def test_spmm_rows_far_longer_than_the_mean(k, dtype, storage):
+    """Rows around the lengths that get a CTA of their own (128, 8 mean rows,
+    4 entries for each of a CTA's lane groups), the first and the last row
+    among them, through the measured choice and the forced row kernels, into a
+    C with more columns than k."""
+    import torch
+
+    rng = np.random.default_rng(k)
+    n = 4000
+    lens = [3000] + [4] * 300 + [127, 128, 129, 130, 255, 256, 257, 512, 513, 1024, 1025, 2049] + [0] * 9
+    lens += [3] * 300 + [1500]
+    rp, c, _ = csr_of_lengths(lens, n, rng)
+    v = (rng.integers(-128, 129, int(rp[-1])) / 64).astype(dtype)
+    m = len(lens)
+    A = pls.SpMat.csr(m, n, rp, c, v)
+    if storage == "bf16":
+        A.set_storage(pls.STORAGE_BF16)
+    ld = (k + 7) // 4 * 4
+    B, C0 = rng.uniform(-1, 1, (n, ld)).astype(dtype), rng.uniform(-1, 1, (m, ld)).astype(dtype)
+    Bd = torch.tensor(B, device="cuda")
+    B64, v64 = np.ascontiguousarray(B[:, :k]).astype(np.float64), v.astype(np.float64)
+    ref = -0.5 * oracle.csr_spmm(rp, c, v64, B64, k) + 0.75 * C0[:, :k]
+    scale = 0.5 * oracle.csr_spmm(rp, c, np.abs(v64), np.abs(B64), k) + 0.75 * np.abs(C0[:, :k].astype(np.float64))
+    for path in (-1, 0, 2):
+        A.set_spmm_path(path)
+        Cd = torch.tensor(C0, device="cuda")
+        torch.cuda.synchronize()
+        A.spmm_dev(Bd.data_ptr(), ld, k, Cd.data_ptr(), ld, -0.5, 0.75)
+        torch.cuda.synchronize()
+        got = Cd.cpu().numpy()
+        check(got[:, :k], ref, scale, 1e-12 if dtype == np.float64 else 1e-5)
+        np.testing.assert_array_equal(got[:, k:], C0[:, k:])
+
+
+def test_spmm_wide_rows_first_call_under_capture():
+    """A first SpMM inside a stream capture (forced row kernel) builds
+    nothing and still computes every row; a later call outside lists them."""
+    import torch
+
+    rng = np.random.default_rng(1)
+    rp, c, v = csr_of_lengths([2000] + [3] * 200, 2500, rng)
+    m, n, k = len(rp) - 1, 2500, 16
+    A = pls.SpMat.csr(m, n, rp, c, v)
+    A.set_spmm_path(0)
+    B = torch.tensor(rng.uniform(-1, 1, (n, k)), device="cuda")
+    ref = oracle.csr_spmm(rp, c, v, B.cpu().numpy(), k)
+    scale = oracle.csr_spmm(rp, c, np.abs(v), np.abs(B.cpu().numpy()), k)
+    C = torch.zeros((m, k), dtype=torch.float64, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        graph.capture_begin(capture_error_mode="thread_local")
+        A.spmm_dev(B.data_ptr(), k, k, C.data_ptr(), k, stream=s.cuda_stream)
+        graph.capture_end()
+    for _ in range(2):
+        C.fill_(7.0)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        check(C.cpu().numpy(), ref, scale, 1e-12)
+    A.spmm_dev(B.data_ptr(), k, k, C.data_ptr(), k)
+    torch.cuda.synchronize()
+    check(C.cpu().numpy(), ref, scale, 1e-12)

@@ -77,6 +77,52 @@ inline DiaRuns dia_runs(const int32_t *offs, int nd) {
   return r;
 }
 
+// What the diagonal-form SpMM with staged values (k_spmm_dia_staged) walks: the runs in ascending
+// order, cut into chunks whose values it holds in shared memory at a time (as
+// many whole runs as keep a 256-thread CTA's 256 / 2^lg_tk units within
+// kDiaSlabBytes: four CTAs share an SM and leave half of it to L1), and the
+// chunks into segments of runs of one length. A unit's slab is unit_bytes: its
+// largest chunk's values, kDiaRows per diagonal, padded to an odd number of
+// 16-byte words so that the units of a warp read different banks.
+constexpr int kDiaSlabBytes = 28 * 1024;
+
+struct DiaWalk {
+  int n_chunks = 0, unit_bytes = 0;
+  int seg0[kDiaMax + 1];   // chunk c: segments [seg0[c], seg0[c + 1])
+  int d0[kDiaMax + 1];     // chunk c: diagonals [d0[c], d0[c + 1])
+  int run0[kDiaMax + 1];   // segment g: runs [run0[g], run0[g + 1])
+  int len[kDiaMax];        // segment g: diagonals per run
+  int o0[kDiaMax];         // run q: first offset
+  int64_t at[kDiaMax];     // run q: first offset * ldb, in elements of B
+};
+
+inline DiaWalk dia_walk(const DiaRuns &runs, int lg_tk, int v_bytes, int64_t ldb) {
+  DiaWalk w{};
+  const int room = kDiaSlabBytes >> (8 - lg_tk);
+  const auto padded = [](int bytes) { return ((bytes + 15) / 16 | 1) * 16; };
+  int nd = 0, segs = 0;  // diagonals in the open chunk, segments so far
+  for (int q = 0; q < runs.n; ++q) {
+    const bool fresh = nd == 0 || padded((nd + runs.len[q]) * kDiaRows * v_bytes) > room;
+    if (fresh) {
+      w.seg0[w.n_chunks] = segs;
+      w.d0[w.n_chunks++] = runs.d0[q];
+      nd = 0;
+    }
+    if (fresh || w.len[segs - 1] != runs.len[q]) {
+      w.run0[segs] = q;
+      w.len[segs++] = runs.len[q];
+    }
+    nd += runs.len[q];
+    w.unit_bytes = std::max(w.unit_bytes, padded(nd * kDiaRows * v_bytes));
+    w.o0[q] = runs.o0[q];
+    w.at[q] = (int64_t)runs.o0[q] * ldb;
+  }
+  w.seg0[w.n_chunks] = segs;
+  w.run0[segs] = runs.n;
+  w.d0[w.n_chunks] = runs.n ? runs.d0[runs.n - 1] + runs.len[runs.n - 1] : 0;
+  return w;
+}
+
 // Line patches of the diagonal-form SpMM (k_spmm_dia). On a grid stencil
 // the runs come one grid line (Ly rows) apart, so the runs of row r at
 // offset +Ly read the rows of B that row r + Ly reads at offset 0. Where the

@@ -31,6 +31,7 @@
 // storage mode change.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -158,44 +159,74 @@ __global__ void k_dia_full(int64_t nblocks, int nd, const V *__restrict__ dv,
   full[b] = bits;
 }
 
-// The RB values of a thread's rows on one diagonal (RB * sizeof(V) bytes:
-// 4, 8 or a multiple of 16, aligned to their size).
-template <int RB, class V>
-__device__ __forceinline__ void ld_rows_vals(const V *p, V (&a)[RB]) {
-  constexpr int bytes = RB * (int)sizeof(V);
-  if constexpr (bytes == 4) {
-    const unsigned t = __ldg(reinterpret_cast<const unsigned *>(p));
-    memcpy(a, &t, 4);
+// The kDiaRows values of one diagonal, from the unit's slab in shared memory
+// or from the diagonal form itself.
+template <bool STAGED, class V>
+__device__ __forceinline__ void ld_diag(const V *p, V (&a)[kDiaRows]) {
+  constexpr int bytes = kDiaRows * (int)sizeof(V);
+  if constexpr (STAGED) {
+    memcpy(a, __builtin_assume_aligned(p, bytes < 16 ? 8 : 16), bytes);
   } else if constexpr (bytes == 8) {
     const uint2 t = __ldg(reinterpret_cast<const uint2 *>(p));
     memcpy(a, &t, 8);
   } else {
-    static_assert(bytes % 16 == 0, "value lines load as whole vectors");
 #pragma unroll
-    for (int i = 0; i < bytes / 16; ++i) {
-      const uint4 t = __ldg(reinterpret_cast<const uint4 *>(p) + i);
-      memcpy(reinterpret_cast<char *>(a) + 16 * i, &t, 16);
+    for (int h = 0; h < bytes / 16; ++h) {
+      const uint4 t = __ldg(reinterpret_cast<const uint4 *>(p) + h);
+      memcpy(reinterpret_cast<char *>(a) + 16 * h, &t, 16);
     }
   }
 }
 
-// One run of len consecutive diagonals for a thread's RB rows: B's rows
-// br0 + j, j = 0 .. RB + len - 2, at bp + j * ldb (columns of the thread's
-// vector); the values of the run's diagonal l at ab + l * kDiaRows (the
-// thread's RB of its block's kDiaRows values).
+// The epilogue of a thread's rows: alpha * sum + beta * C.
+template <class X, class Acc, int VEC>
+__device__ __forceinline__ void dia_store(X *C, int64_t ldc, int64_t r0, int64_t m, int kk,
+                                          X alpha, X beta, int beta_nz,
+                                          const Acc (&acc)[kDiaRows][VEC]) {
+#pragma unroll
+  for (int i = 0; i < kDiaRows; ++i) {
+    const int64_t r = r0 + i;
+    if (r < m) {
+      X *cp = C + r * ldc + kk;
+      X out[VEC];
+      if (beta_nz) {
+        X old[VEC];
+        ld_vec_plain<X, VEC>(cp, old);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+          out[v] = (X)acc[i][v] * alpha + beta * old[v];
+      } else {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+          out[v] = (X)acc[i][v] * alpha;
+      }
+      st_vec<X, VEC>(cp, out);
+    }
+  }
+}
+
+// Threads of both kernels: (unit of kDiaRows rows) x (TK = 2^lg_tk lanes, one
+// 16-byte vector of C's columns each); a thread loops over C's columns in steps
+// of TK * VEC. A thread's unit comes from the line-patch plan (dia_patch_plan /
+// dia_patch_unit in dia_plan.hpp).
+
+// ---- values from global memory (few lanes per unit) ---------------------
+//
+// One run of len consecutive diagonals for a thread's kDiaRows rows: B's rows
+// br0 + j, j = 0 .. kDiaRows + len - 2, at bp + j * ldb (columns of the
+// thread's vector); the values of the run's diagonal l at ab + l * kDiaRows.
 // INSIDE: len == kDiaRun and the rows all lie inside B, so the loads are
 // neither checked nor predicated (otherwise rows outside [0, n) read as
-// zeros). CHECK: absent entries are skipped (without it the block must store
-// every diagonal). Either way each stored entry is one fma in ascending
-// diagonal order.
-template <bool INSIDE, bool CHECK, int RB, class V, class X, class Acc, int VEC>
-__device__ __forceinline__ void dia_run(const X *bp, int64_t ldb, int64_t br0, int64_t n,
-                                        int len, const V *ab, Acc (&acc)[RB][VEC]) {
-  constexpr bool FAST = INSIDE;
-  X bv[RB + kDiaRun - 1][VEC];
+// zeros). Absent entries are skipped; each stored entry is one fma in
+// ascending diagonal order.
+template <bool INSIDE, class V, class X, class Acc, int VEC>
+__device__ __forceinline__ void dia_run_direct(const X *bp, int64_t ldb, int64_t br0,
+                                               int64_t n, int len, const V *ab,
+                                               Acc (&acc)[kDiaRows][VEC]) {
+  X bv[kDiaRows + kDiaRun - 1][VEC];
 #pragma unroll
-  for (int j = 0; j < RB + kDiaRun - 1; ++j) {
-    if (FAST || (j < RB + len - 1 && br0 + j >= 0 && br0 + j < n)) {
+  for (int j = 0; j < kDiaRows + kDiaRun - 1; ++j) {
+    if (INSIDE || (j < kDiaRows + len - 1 && br0 + j >= 0 && br0 + j < n)) {
       ld_vec<X, VEC>(bp + j * ldb, bv[j]);
     } else {
 #pragma unroll
@@ -205,12 +236,12 @@ __device__ __forceinline__ void dia_run(const X *bp, int64_t ldb, int64_t br0, i
   }
 #pragma unroll
   for (int l = 0; l < kDiaRun; ++l) {
-    if (FAST || l < len) {
-      V a[RB];
-      ld_rows_vals<RB, V>(ab + l * kDiaRows, a);
+    if (INSIDE || l < len) {
+      V a[kDiaRows];
+      ld_diag<false, V>(ab + l * kDiaRows, a);
 #pragma unroll
-      for (int i = 0; i < RB; ++i)
-        if (!CHECK || !dia_absent(a[i])) {
+      for (int i = 0; i < kDiaRows; ++i)
+        if (!dia_absent(a[i])) {
           const Acc ai = to_acc<Acc>(a[i]);
 #pragma unroll
           for (int v = 0; v < VEC; ++v)
@@ -220,41 +251,22 @@ __device__ __forceinline__ void dia_run(const X *bp, int64_t ldb, int64_t br0, i
   }
 }
 
-// Line patches: dia_patch_plan / dia_patch_unit in dia_plan.hpp.
-
-// Rows per thread. Each thread owns kDiaThreadRows consecutive rows of one
-// block of kDiaRows (a unit) and one 16-byte vector of C's columns.
-constexpr int kDiaThreadRows = 4;
-
-// Threads: (unit of RB rows) x (TK column vectors of VEC); a thread loops
-// over C's columns in steps of TK * VEC. MASK (threads that make more than
-// one pass over the columns): the block's full-diagonal mask is loaded first
-// and blocks that store every diagonal skip the absent checks; with one pass
-// that load's latency costs more than the checks (C3, FP64: 0.233 against
-// 0.331 ms at k = 8, 0.725 against 0.849 ms at k = 32; at k = 128, two
-// passes, 2.21 against 2.43 ms). A thread's unit comes from the line-patch
-// plan (dia_patch_unit).
-template <class V, class X, int VEC, bool MASK, int RB>
-__global__ void __launch_bounds__(256, RB == kDiaRows ? 4 : 6)
+template <class V, class X, int VEC>
+__global__ void __launch_bounds__(256, 4)
     k_spmm_dia(int32_t m, int32_t n, int nd, DiaRuns runs, const V *__restrict__ dv,
-               const uint32_t *__restrict__ dfull, uint32_t full_mask,
                const X *__restrict__ B, int64_t ldb, X *__restrict__ C, int64_t ldc, int k,
                int lg_tk, DiaPatchPlan patch, X alpha, X beta, int beta_nz) {
-  static_assert(kDiaRows % RB == 0, "a thread's rows lie in one block");
-  constexpr int SUB = kDiaRows / RB;  // units per block
   using Acc = typename AccOf<V, X>::type;
   const int64_t u = dia_patch_unit(blockIdx.x, (int)threadIdx.x, lg_tk, patch);
   const int tk = (int)(threadIdx.x & ((1 << lg_tk) - 1));
-  const int64_t r0 = u * RB;
+  const int64_t r0 = u * kDiaRows;
   if (r0 >= m)
     return;
-  const int64_t rb = u / SUB;  // the unit's block
-  const V *ab = dv + rb * nd * kDiaRows + (u % SUB) * RB;
-  const bool full = MASK && (__ldg(dfull + rb) & full_mask) == full_mask;
+  const V *ab = dv + u * nd * kDiaRows;
   for (int kk = tk * VEC; kk < k; kk += VEC << lg_tk) {
-    Acc acc[RB][VEC];
+    Acc acc[kDiaRows][VEC];
 #pragma unroll
-    for (int i = 0; i < RB; ++i)
+    for (int i = 0; i < kDiaRows; ++i)
 #pragma unroll
       for (int v = 0; v < VEC; ++v)
         acc[i][v] = Acc(0);
@@ -263,35 +275,203 @@ __global__ void __launch_bounds__(256, RB == kDiaRows ? 4 : 6)
       const int64_t br0 = r0 + o0;
       const X *bp = B + br0 * ldb + kk;
       const V *aq = ab + runs.d0[q] * kDiaRows;
-      if (len == kDiaRun && br0 >= 0 && br0 + RB + kDiaRun - 2 < n) {
-        if (MASK && full)
-          dia_run<true, false, RB, V, X, Acc, VEC>(bp, ldb, br0, n, len, aq, acc);
-        else
-          dia_run<true, true, RB, V, X, Acc, VEC>(bp, ldb, br0, n, len, aq, acc);
+      if (len == kDiaRun && br0 >= 0 && br0 + kDiaRows + kDiaRun - 2 < n)
+        dia_run_direct<true, V, X, Acc, VEC>(bp, ldb, br0, n, len, aq, acc);
+      else
+        dia_run_direct<false, V, X, Acc, VEC>(bp, ldb, br0, n, len, aq, acc);
+    }
+    dia_store<X, Acc, VEC>(C, ldc, r0, m, kk, alpha, beta, beta_nz, acc);
+  }
+}
+
+// ---- values staged in shared memory ---------------------------------------
+
+// acc[v] = fma(a, b[v], acc[v]) unless the stored value is the reserved
+// pattern: one compare and predicated FMAs (a select per element otherwise).
+__device__ __forceinline__ void fma_stored(double s, const double (&b)[2], double (&acc)[2]) {
+  asm("{ .reg .pred p; setp.ne.s32 p, %5, %6;\n\t"
+      "@p fma.rn.f64 %0, %2, %3, %0;\n\t@p fma.rn.f64 %1, %2, %4, %1; }"
+      : "+d"(acc[0]), "+d"(acc[1])
+      : "d"(s), "d"(b[0]), "d"(b[1]), "r"(__double2hiint(s)), "n"((int)(kAbsentD >> 32)));
+}
+__device__ __forceinline__ void fma_pred(int bits, int absent, float s, const float (&b)[4],
+                                         float (&acc)[4]) {
+  asm("{ .reg .pred p; setp.ne.s32 p, %9, %10;\n\t"
+      "@p fma.rn.f32 %0, %4, %5, %0;\n\t@p fma.rn.f32 %1, %4, %6, %1;\n\t"
+      "@p fma.rn.f32 %2, %4, %7, %2;\n\t@p fma.rn.f32 %3, %4, %8, %3; }"
+      : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+      : "f"(s), "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(b[3]), "r"(bits), "r"(absent));
+}
+__device__ __forceinline__ void fma_pred(int bits, int absent, float s, const float (&b)[2],
+                                         float (&acc)[2]) {
+  asm("{ .reg .pred p; setp.ne.s32 p, %5, %6;\n\t"
+      "@p fma.rn.f32 %0, %2, %3, %0;\n\t@p fma.rn.f32 %1, %2, %4, %1; }"
+      : "+f"(acc[0]), "+f"(acc[1])
+      : "f"(s), "f"(b[0]), "f"(b[1]), "r"(bits), "r"(absent));
+}
+template <int VEC>
+__device__ __forceinline__ void fma_stored(float s, const float (&b)[VEC], float (&acc)[VEC]) {
+  fma_pred(__float_as_int(s), (int)kAbsentF, s, b, acc);
+}
+template <int VEC>
+__device__ __forceinline__ void fma_stored(__nv_bfloat16 s, const float (&b)[VEC],
+                                           float (&acc)[VEC]) {
+  fma_pred((int)__bfloat16_as_ushort(s), (int)kAbsentH, __bfloat162float(s), b, acc);
+}
+
+// What a run can rely on: kFull every entry is stored and every row lies in B;
+// kInside every row lies in B; kEdge neither.
+constexpr int kFull = 0, kInside = 1, kEdge = 2;
+
+// One run of LEN consecutive diagonals for a thread's kDiaRows rows: B's rows
+// j = 0 .. kDiaRows + LEN - 2 at base + at[j] (base is the run's, the same for
+// the whole warp), the run's values at `a`, kDiaRows per diagonal, one fma per
+// entry in ascending diagonal order. Absent entries are skipped unless kFull;
+// with kEdge a row outside B (row br0 + j outside [0, n)), whose entries are
+// all absent, reads row 0 of B (at `safe`) instead.
+template <int LEN, int MODE, class V, class X, class Acc, int VEC, class Off>
+__device__ __forceinline__ void dia_run(const X *base, const Off (&at)[kDiaRows + kDiaRun - 1],
+                                        int64_t br0, int64_t n, const X *safe, const V *a,
+                                        Acc (&acc)[kDiaRows][VEC]) {
+  X bv[kDiaRows + LEN - 1][VEC];
+#pragma unroll
+  for (int j = 0; j < kDiaRows + LEN - 1; ++j) {
+    const X *p = base + at[j];
+    if (MODE == kEdge && (br0 + j < 0 || br0 + j >= n))
+      p = safe;
+    ld_vec<X, VEC>(p, bv[j]);
+  }
+#pragma unroll
+  for (int l = 0; l < LEN; ++l) {
+    V av[kDiaRows];
+    ld_diag<true, V>(a + l * kDiaRows, av);
+#pragma unroll
+    for (int i = 0; i < kDiaRows; ++i) {
+      Acc b[VEC];
+#pragma unroll
+      for (int v = 0; v < VEC; ++v)
+        b[v] = to_acc<Acc>(bv[i + l][v]);
+      if constexpr (MODE == kFull) {
+        const Acc ai = to_acc<Acc>(av[i]);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+          acc[i][v] = fma(ai, b[v], acc[i][v]);
       } else {
-        dia_run<false, true, RB, V, X, Acc, VEC>(bp, ldb, br0, n, len, aq, acc);
+        fma_stored(av[i], b, acc[i]);
       }
     }
+  }
+}
+
+// Piece of the values a lane copies at a time: 16 bytes (a diagonal's
+// kDiaRows FP32 values, half of its FP64 ones), or its 8 for BF16.
+template <class V> struct DiaPiece { using T = uint4; };
+template <> struct DiaPiece<__nv_bfloat16> { using T = uint2; };
+
+// The TK lanes of a unit first copy its values, coalesced, into the unit's
+// slab of shared memory (in chunks of whole runs where all of them take too
+// much, dia_walk), and learn on the way whether an entry is absent. The inner
+// loop then waits for B's rows alone, once per run, and units that store
+// every entry run without absent checks.
+//
+// Bound by the L1 data pipe (70% of its peak on the 27-point stencil at FP64
+// k = 32; B's rows cross it 13.5 times) and by the latency of B's rows.
+// Measured against the kernel above (27-point stencil unless said otherwise):
+// FP64 128^3 k = 32 694 -> 510 us, 80^3 k = 128 527 -> 393 us, 95^3 k = 40
+// 500 -> 352 us, 96^3 k = 16 178 -> 134 us; FP32 128^3 k = 32 256 -> 240 us;
+// BF16 values, 95^3 k = 128 366 -> 320 us; FP64 band of 15, 300,000 rows,
+// k = 64 117 -> 90 us. More CTAs per SM (5 or 6, 48 or 40 registers) or fewer
+// (3) were slower: 811, 751 and 781 us at k = 32.
+template <class V, class X, int VEC, class Off>
+__global__ void __launch_bounds__(256, 4)
+    k_spmm_dia_staged(int32_t m, int32_t n, int nd, const __grid_constant__ DiaWalk w,
+                      const V *__restrict__ dv, const X *__restrict__ B, int64_t ldb,
+                      X *__restrict__ C, int64_t ldc, int k, int lg_tk, DiaPatchPlan patch,
+                      X alpha, X beta, int beta_nz) {
+  using Acc = typename AccOf<V, X>::type;
+  using Piece = typename DiaPiece<V>::T;
+  constexpr int PV = (int)(sizeof(Piece) / sizeof(V));  // values per piece
+  extern __shared__ uint4 dia_slab[];
+  const int64_t u = dia_patch_unit(blockIdx.x, (int)threadIdx.x, lg_tk, patch);
+  const int tk = (int)(threadIdx.x & ((1 << lg_tk) - 1));
+  V *const slab = reinterpret_cast<V *>(reinterpret_cast<char *>(dia_slab) +
+                                        (threadIdx.x >> lg_tk) * w.unit_bytes);
+  const int64_t r0 = u * kDiaRows;
+  const bool live = r0 < m;
+  const V *const ab = dv + u * nd * kDiaRows;
+  const int last = w.run0[w.seg0[w.n_chunks]] - 1;
+  // every run's rows of the unit lie in B
+  const bool inside = live && r0 + w.o0[0] >= 0 &&
+                      r0 + w.o0[last] + w.len[w.seg0[w.n_chunks] - 1] + kDiaRows - 2 < n;
+  int mode = kEdge;
+  for (int k0 = 0; k0 < k; k0 += VEC << lg_tk) {
+    const int kk = k0 + tk * VEC;
+    const bool act = live && kk < k;
+    // lanes past the last column read column 0 of their rows and store nothing
+    const int kc = kk < k ? kk : 0;
+    Off at[kDiaRows + kDiaRun - 1];
 #pragma unroll
-    for (int i = 0; i < RB; ++i) {
-      const int64_t r = r0 + i;
-      if (r < m) {
-        X *cp = C + r * ldc + kk;
-        X out[VEC];
-        if (beta_nz) {
-          X old[VEC];
-          ld_vec_plain<X, VEC>(cp, old);
+    for (int j = 0; j < kDiaRows + kDiaRun - 1; ++j)
+      at[j] = (Off)((r0 + j) * ldb + kc);
+    Acc acc[kDiaRows][VEC];
 #pragma unroll
-          for (int v = 0; v < VEC; ++v)
-            out[v] = (X)acc[i][v] * alpha + beta * old[v];
-        } else {
+    for (int i = 0; i < kDiaRows; ++i)
 #pragma unroll
-          for (int v = 0; v < VEC; ++v)
-            out[v] = (X)acc[i][v] * alpha;
+      for (int v = 0; v < VEC; ++v)
+        acc[i][v] = Acc(0);
+    for (int c = 0; c < w.n_chunks; ++c) {
+      const int d0 = w.d0[c];
+      if (w.n_chunks > 1 || k0 == 0) {
+        __syncwarp();  // the chunk before is read
+        bool absent = false;
+        if (live) {
+          const Piece *src = reinterpret_cast<const Piece *>(ab + d0 * kDiaRows);
+          const int pieces = (w.d0[c + 1] - d0) * kDiaRows / PV;
+#pragma unroll 4
+          for (int i = tk; i < pieces; i += 1 << lg_tk) {
+            const Piece t = __ldcs(src + i);
+            V tv[PV];
+            memcpy(tv, &t, sizeof(t));
+#pragma unroll
+            for (int p = 0; p < PV; ++p)
+              absent = absent || dia_absent(tv[p]);
+            reinterpret_cast<Piece *>(slab)[i] = t;
+          }
         }
-        st_vec<X, VEC>(cp, out);
+        const bool edges = __any_sync(0xffffffffu, !inside);
+        mode = edges ? kEdge : __any_sync(0xffffffffu, absent) ? kInside : kFull;
+        __syncwarp();
+      }
+      const V *a = slab;
+      for (int g = w.seg0[c]; g < w.seg0[c + 1]; ++g) {
+        const auto seg = [&](auto len_tag, auto mode_tag) {
+          constexpr int LEN = decltype(len_tag)::value;
+          constexpr int MODE = decltype(mode_tag)::value;
+#pragma unroll 1
+          for (int q = w.run0[g]; q < w.run0[g + 1]; ++q) {
+            dia_run<LEN, MODE, V, X, Acc, VEC, Off>(B + w.at[q], at, r0 + w.o0[q], n, B + kc, a,
+                                                    acc);
+            a += LEN * kDiaRows;
+          }
+        };
+        const auto by_len = [&](auto mode_tag) {
+          if (w.len[g] == 3)
+            seg(std::integral_constant<int, 3>{}, mode_tag);
+          else if (w.len[g] == 2)
+            seg(std::integral_constant<int, 2>{}, mode_tag);
+          else
+            seg(std::integral_constant<int, 1>{}, mode_tag);
+        };
+        if (mode == kFull)
+          by_len(std::integral_constant<int, kFull>{});
+        else if (mode == kInside)
+          by_len(std::integral_constant<int, kInside>{});
+        else if (live)
+          by_len(std::integral_constant<int, kEdge>{});
       }
     }
+    if (act)
+      dia_store<X, Acc, VEC>(C, ldc, r0, m, kk, alpha, beta, beta_nz, acc);
   }
 }
 
@@ -378,16 +558,28 @@ void dia_launch(const CsrDev &c, int32_t m, const X *B, int64_t ldb, X *C, int64
   int lg_tk = 0;
   while ((1 << lg_tk) < cols && lg_tk < 5)
     ++lg_tk;
-  constexpr int RB = kDiaThreadRows;
-  const int64_t nunits = div_up(m, RB);
+  const int64_t nunits = div_up(m, kDiaRows);
   const int64_t threads = nunits << lg_tk;
-  const uint32_t full_mask = d.nd >= 32 ? 0xffffffffu : (1u << d.nd) - 1u;
-  const bool passes = cols > (1 << lg_tk);
-  const DiaPatchPlan patch = dia_patch_plan(runs, RB, nunits, lg_tk);
-  auto kern = passes ? k_spmm_dia<V, X, VEC, true, RB> : k_spmm_dia<V, X, VEC, false, RB>;
-  kern<<<(unsigned)div_up(threads, 256), 256, 0, s>>>(
-      m, c.ncols, d.nd, runs, d.vals.as<V>(), d.full.as<uint32_t>(), full_mask, B, ldb, C, ldc,
-      k, lg_tk, patch, alpha, beta, beta != X(0));
+  const DiaPatchPlan patch = dia_patch_plan(runs, kDiaRows, nunits, lg_tk);
+  const unsigned grid = (unsigned)div_up(threads, 256);
+  // Staging pays from 8 lanes per unit on, where the direct kernel loads each
+  // value in every lane: staged against direct, FP64 96^3 k = 16 (8 lanes)
+  // 134 / 168 us, FP32 128^3 k = 32 (8 lanes) 240 / 256 us; FP64 128^3 k = 8
+  // (4 lanes) 231 / 230 us, FP32 k = 8 (2 lanes) 176 / 157 us.
+  if (lg_tk < 3) {
+    k_spmm_dia<V, X, VEC><<<grid, 256, 0, s>>>(m, c.ncols, d.nd, runs, d.vals.as<V>(), B, ldb, C,
+                                               ldc, k, lg_tk, patch, alpha, beta, beta != X(0));
+  } else {
+    const DiaWalk w = dia_walk(runs, lg_tk, (int)sizeof(V), ldb);
+    // 32-bit element offsets into B: the unit's rows and those after them that
+    // a run reads, before the run's own offset.
+    const bool off32 = ((int64_t)m + 2 * kDiaRows + kDiaRun) * ldb < (int64_t)UINT32_MAX;
+    auto kern =
+        off32 ? k_spmm_dia_staged<V, X, VEC, uint32_t> : k_spmm_dia_staged<V, X, VEC, uint64_t>;
+    kern<<<grid, 256, (size_t)w.unit_bytes << (8 - lg_tk), s>>>(
+        m, c.ncols, d.nd, w, d.vals.as<V>(), B, ldb, C, ldc, k, lg_tk, patch, alpha, beta,
+        beta != X(0));
+  }
   PLS_LAUNCH_CHECK();
 }
 

@@ -212,3 +212,103 @@ def test_spmm_wide_rows_first_call_under_capture():
     A.spmm_dev(B.data_ptr(), k, k, C.data_ptr(), k)
     torch.cuda.synchronize()
     check(C.cpu().numpy(), ref, scale, 1e-12)
+
+
+# ------------------------------------------------------ diagonal-form SpMM
+
+
+def stencil_2d9(nx, ny, rng):
+    """9-point stencil on an nx x ny grid: three runs of three diagonals."""
+    i = np.arange(nx * ny)
+    x, y = i % nx, i // nx
+    cols, mask = [], []
+    for dy in (-1, 0, 1):
+        for dx in (-1, 0, 1):
+            cols.append(i + dy * nx + dx)
+            mask.append((x + dx >= 0) & (x + dx < nx) & (y + dy >= 0) & (y + dy < ny))
+    cols, mask = np.stack(cols, 1), np.stack(mask, 1)
+    rp = np.zeros(nx * ny + 1, np.int32)
+    rp[1:] = np.cumsum(mask.sum(1))
+    return nx * ny, nx * ny, rp, cols[mask].astype(np.int32), rng.standard_normal(int(rp[-1]))
+
+
+def dia_matrix(name, rng):
+    if name == "stencil27":
+        return W.stencil_27pt(11, seed=3)
+    if name == "laplace":
+        return W.laplacian_2d(23)
+    if name == "lines":  # lines of 64 rows: line patches
+        return stencil_2d9(64, 40, rng)
+    if name == "band15":  # 31 consecutive diagonals: the last run is one diagonal
+        return W.banded_csr(301, 15, rng)
+    m, n = (260, 400) if name == "wide" else (403, 250)  # a band in a matrix that is not square
+    r = np.repeat(np.arange(m), 5)
+    c = r + np.tile(np.array([-2, -1, 0, 1, 6]), m)
+    keep = (c >= 0) & (c < n)
+    rp = np.zeros(m + 1, np.int32)
+    rp[1:] = np.cumsum(np.bincount(r[keep], minlength=m))
+    return m, n, rp, c[keep].astype(np.int32), rng.standard_normal(int(rp[-1]))
+
+
+@pytest.mark.parametrize("name", ["stencil27", "laplace", "lines", "band15", "wide", "tall"])
+@pytest.mark.parametrize("dtype,storage", [(np.float64, "native"), (np.float64, "fp32"), (np.float64, "bf16"),
+                                           (np.float32, "native"), (np.float32, "bf16")])
+def test_diagonal_form_equals_row_kernel_at_every_lane_count(name, dtype, storage):
+    """1 to 32 lanes per unit, lanes past the last column, one and several
+    passes over the columns, values in one and in several chunks: the bits of
+    the row kernel, with NaN and infinities in rows of B that only some rows
+    of A read, and with beta."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    m, n, rp, c, v = dia_matrix(name, rng)
+    A = pls.SpMat.csr(m, n, rp, c, v.astype(dtype))
+    A.set_storage({"native": pls.STORAGE_NATIVE, "fp32": pls.STORAGE_FP32, "bf16": pls.STORAGE_BF16}[storage])
+    vec = 16 // np.dtype(dtype).itemsize
+    for k in (vec, 2 * vec, 3 * vec, 8 * vec, 13 * vec, 16 * vec, 32 * vec, 41 * vec):
+        B = rng.uniform(-1, 1, (n, k + vec)).astype(dtype)
+        B[n // 2, :] = np.nan
+        B[n // 3, 1] = np.inf
+        B[0, 0] = -np.inf
+        B[n - 1, k - 1] = np.nan
+        C0 = rng.uniform(-1, 1, (m, k + vec)).astype(dtype)
+        Bd = torch.tensor(B, device="cuda")
+        for alpha, beta in ((1.0, 0.0), (-0.5, 2.0)):
+            out = []
+            for path in (0, 3):
+                A.set_spmm_path(path)
+                Cd = torch.tensor(C0, device="cuda")
+                torch.cuda.synchronize()
+                A.spmm_dev(Bd.data_ptr(), k + vec, k, Cd.data_ptr(), k + vec, alpha, beta)
+                torch.cuda.synchronize()
+                assert A.spmm_info()["path"] == path
+                out.append(Cd.cpu().numpy())
+            np.testing.assert_array_equal(np.isnan(out[0]), np.isnan(out[1]), err_msg=str(k))
+            if beta == 0 and k > 2 * vec:
+                np.testing.assert_array_equal(out[0], out[1], err_msg=str(k))
+            else:  # up to two vectors the row kernel adds in a tree; its beta * C may be fused
+                tol = 1e-13 if dtype == np.float64 and storage == "native" else 1e-4  # of sums of 31 terms
+                fin = np.isfinite(out[0])
+                np.testing.assert_array_equal(out[0][~fin], out[1][~fin])
+                np.testing.assert_allclose(out[0][fin], out[1][fin], rtol=tol, atol=tol)
+
+
+def test_diagonal_form_beyond_32_bit_offsets():
+    """Rows of B and C 65,600 elements apart: offsets past 2^32 elements."""
+    import torch
+
+    m, ld, k = 65_700, 65_600, 32  # staged values
+    rng = np.random.default_rng(2)
+    _, _, rp, c, v = W.banded_csr(m, 1, rng)
+    A = pls.SpMat.csr(m, m, rp, c, v.astype(np.float32))
+    A.set_spmm_path(3)
+    B = torch.empty((m, ld), dtype=torch.float32, device="cuda")
+    B[:, :k] = torch.tensor(rng.uniform(-1, 1, (m, k)).astype(np.float32), device="cuda")
+    C = torch.empty((m, k), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    A.spmm_dev(B.data_ptr(), ld, k, C.data_ptr(), k)
+    torch.cuda.synchronize()
+    assert A.spmm_info()["path"] == 3
+    B64 = B[:, :k].double().cpu().numpy()
+    v64 = v.astype(np.float32).astype(np.float64)
+    check(C.cpu().numpy(), oracle.csr_spmm(rp, c, v64, B64, k), oracle.csr_spmm(rp, c, np.abs(v64), np.abs(B64), k), 1e-6)

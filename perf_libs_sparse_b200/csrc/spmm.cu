@@ -467,8 +467,19 @@ __device__ __forceinline__ void ld_block_line(const V *p, V (&a)[BS]) {
 // lanes), then adds, for every row i of the block, a_ij * B_j in ascending
 // j: per element of C the order of the scalar kernel above, blocks in stored
 // order and columns of a block ascending, so the results are the same bits.
+//
+// Bound by the latency of B's rows. Blocks of 8 are held to two CTAs per SM
+// rather than to what the compiler picks (92 registers, two CTAs as well):
+// the 128 registers that two leave room for let it load a block's rows of B
+// and its values together. Measured (32,768 x 8 random blocks, k = 128): BF16
+// values 193 -> 168 us, FP32 242 -> 186 us, FP64 (16,384 block rows, k = 64)
+// 152 -> 113 us; three CTAs (80 registers) 187 / 189 / 125 us, one (151)
+// 168 / 260 / 143 us. FP64 B and C with reduced values (FP32 sums, half the
+// accumulators) gain nothing from it (24.6 against 24.9 us, 2,652 x 5 blocks,
+// k = 122), and blocks of 2 and 4 run best as compiled.
 template <int BS, bool RM, class V, class X, int VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(
+    256, BS == 8 && sizeof(X) == sizeof(typename AccOf<V, X>::type) ? 2 : 0)
     k_spmm_bsr_vec(int32_t mb, const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                    const V *__restrict__ val, const X *__restrict__ B, int64_t ldb,
                    X *__restrict__ C, int64_t ldc, int k, int lg_tk, X alpha, X beta,

@@ -57,6 +57,14 @@ struct InstDesc {
   // copy made at creation; staged rows read them instead of the packed
   // entries (null otherwise)
   const float *band_val;
+  // The same by blocks of 4 rows, where the rows' columns overlap enough: for
+  // every block, band_w float4s, one per column from the block's first, with
+  // the 4 rows' values in that column; the blocks a warp takes together,
+  // band_p of them, side by side in each column. And every row's first and
+  // last column.
+  const float4 *band_blk;
+  const int2 *band_rng;
+  int32_t band_w, band_p;
 };
 
 struct Item {
@@ -76,24 +84,56 @@ constexpr int kBatchThreads = 256;
 constexpr int kStageFloats = 8192;  // 32 KB of shared memory per CTA
 constexpr int kStageCols = 32;      // widest column slice of a staged item
 
-// One item's rows with the instance's vector shape.
-template <class Rows, bool OFF32>
-__device__ __forceinline__ void batch_rows(const Rows &A, const InstDesc &d, const Item &w,
-                                           int lane, float alpha, float beta, int beta_nz,
+// An instance's rows with the current row's range already loaded.
+struct PackedRowsAt {
+  using V = float;
+  const int2 *cv;
+  int32_t s, e;
+  __device__ __forceinline__ bool range(int64_t, int32_t &rs, int32_t &re, int32_t &aux) const {
+    rs = s;
+    re = e;
+    aux = 0;
+    return true;
+  }
+  __device__ __forceinline__ void entry(int32_t q, int32_t, int32_t &c, float &a,
+                                        const L2Policy &pol) const {
+    const int2 t = ld_stream(cv + q, pol.stream);
+    c = t.x;
+    a = __int_as_float(t.y);
+  }
+};
+
+// One item's rows with the instance's vector shape, the next rows' ranges
+// loaded while these are computed.
+template <bool OFF32>
+__device__ __forceinline__ void batch_rows(const InstDesc &d, const Item &w, int lane,
+                                           float alpha, float beta, int beta_nz,
                                            const L2Policy &pol) {
-  const int lg_g = d.lg_tk + d.lg_tn;
-  for (int32_t r0 = w.row0; r0 < w.row1; r0 += (32 >> lg_g)) {
-    const int32_t row = r0 + (lane >> lg_g);
+  const int lg_g = d.lg_tk + d.lg_tn, step = 32 >> lg_g;
+  int32_t row = w.row0 + (lane >> lg_g);
+  PackedRowsAt A{d.cv, 0, 0};
+  if (row < w.row1) {
+    A.s = __ldg(d.rp + row);
+    A.e = __ldg(d.rp + row + 1);
+  }
+  for (int32_t r0 = w.row0; r0 < w.row1; r0 += step, row += step) {
     const bool live = row < w.row1;
+    int32_t ns = 0, ne = 0;
+    if (row + step < w.row1) {
+      ns = __ldg(d.rp + row + step);
+      ne = __ldg(d.rp + row + step + 1);
+    }
     if (d.path == 0)
-      spmm_row_group<4, 1, float, float, Rows, OFF32, kEntriesAhead>(
+      spmm_row_group<4, 1, float, float, PackedRowsAt, OFF32, kEntriesAhead>(
           A, row, live, d.lg_tk, d.lg_tn, d.B, d.ldb, d.C, d.ldc, d.k, alpha, beta, beta_nz, pol);
     else if (d.path == 1)
-      spmm_row_group<1, 1, float, float, Rows, OFF32, kEntriesAhead>(
+      spmm_row_group<1, 1, float, float, PackedRowsAt, OFF32, kEntriesAhead>(
           A, row, live, d.lg_tk, d.lg_tn, d.B, d.ldb, d.C, d.ldc, d.k, alpha, beta, beta_nz, pol);
     else
-      spmm_row_group<1, 2, float, float, Rows, OFF32, kEntriesAhead>(
+      spmm_row_group<1, 2, float, float, PackedRowsAt, OFF32, kEntriesAhead>(
           A, row, live, d.lg_tk, d.lg_tn, d.B, d.ldb, d.C, d.ldc, d.k, alpha, beta, beta_nz, pol);
+    A.s = ns;
+    A.e = ne;
   }
 }
 
@@ -158,6 +198,42 @@ __device__ __forceinline__ void batch_bsr_rows(const InstDesc &d, const Item &w,
   }
 }
 
+// Float4s from one window row to the next in the stage, for tk lanes per row:
+// one more for 2 and 4 lanes, so that the row groups of a quarter warp, which
+// read rows 4 apart, do not start in the same banks.
+__host__ __device__ constexpr int stage_stride(int tk) { return tk == 2 || tk == 4 ? tk + 1 : tk; }
+
+// Lanes per row of an instance's first (widest) column slice.
+__host__ __device__ constexpr int stage_lanes(int k) {
+  return k < 1 ? 1 : ((k < kStageCols ? k : kStageCols) + 3) / 4;
+}
+
+// The columns of a block of 4 rows (first row 4 * blk) with consecutive
+// columns: each row's range, the block's range [lo, hi] and the columns
+// [lo_all, hi_all] that every row stores.
+struct BandBlock {
+  int2 row[4];
+  int lo, hi, lo_all, hi_all;
+};
+__device__ __forceinline__ BandBlock band_block(const int2 *__restrict__ rng, int32_t m,
+                                                int32_t blk) {
+  BandBlock b;
+  b.lo = INT32_MAX, b.hi = -1, b.lo_all = 0, b.hi_all = INT32_MAX;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    b.row[i] = 4 * blk + i < m ? __ldg(rng + 4 * blk + i) : make_int2(0, -1);
+    if (b.row[i].y >= b.row[i].x) {
+      b.lo = min(b.lo, b.row[i].x);
+      b.hi = max(b.hi, b.row[i].y);
+    }
+    b.lo_all = max(b.lo_all, b.row[i].x);
+    b.hi_all = min(b.hi_all, b.row[i].y);
+  }
+  if (b.hi < 0)
+    b.lo = 0;  // no entries
+  return b;
+}
+
 // One staged item, by the whole CTA. The window of B (rows lo .. lo + w - 1,
 // columns c0 .. c0 + ks - 1) is copied into `stage` (row stride 4 tk
 // floats); then tk lanes per row own 4 columns each, and every row of the
@@ -170,7 +246,7 @@ __device__ __forceinline__ void staged_item(const SItem &w, const InstDesc &d,
                                             int beta_nz) {
   constexpr int warps = kBatchThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int TK = w.tk, KSP = 4 * w.tk;
+  const int TK = w.tk, KSP = 4 * w.tk, S = stage_stride(w.tk);
   if ((d.ldb & 3) == 0 && ((uintptr_t)d.B & 15) == 0) {
     // TK lanes per window row, a float4 each (c0 is a multiple of 32, so
     // every row segment starts on 16 bytes)
@@ -191,7 +267,7 @@ __device__ __forceinline__ void staged_item(const SItem &w, const InstDesc &d,
           v.z = c + 2 < w.ks ? __ldg(p + 2) : 0.f;
           v.w = 0.f;  // c + 3 >= ks here
         }
-        dst[r * TK] = v;
+        dst[r * S] = v;
       }
     }
   } else {
@@ -203,7 +279,7 @@ __device__ __forceinline__ void staged_item(const SItem &w, const InstDesc &d,
       const float *src = d.B + (int64_t)w.lo * d.ldb + w.c0 + (in ? c : 0);
 #pragma unroll 4
       for (int r = warp * per + rs; r < w.w; r += warps * per)
-        stage[r * KSP + c] = in ? __ldg(src + (int64_t)r * d.ldb) : 0.f;
+        stage[r * 4 * S + c] = in ? __ldg(src + (int64_t)r * d.ldb) : 0.f;
     }
   }
   __syncthreads();
@@ -215,55 +291,8 @@ __device__ __forceinline__ void staged_item(const SItem &w, const InstDesc &d,
   const int kk = w.c0 + 4 * tk;  // this lane's first column of C
   const int kend = w.c0 + w.ks;
   const bool vec = d.path == 0 && kk + 4 <= kend;
-  for (int32_t row = w.row0 + warp * per + rs; row < w.row1; row += warps * per) {
-    const int32_t s = __ldg(d.rp + row), e = __ldg(d.rp + row + 1);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    const auto add = [&](int2 t) {
-      const float4 b = st4[(t.x - w.lo) * TK + tk];
-      const float a = __int_as_float(t.y);
-      acc.x = fmaf(a, b.x, acc.x);
-      acc.y = fmaf(a, b.y, acc.y);
-      acc.z = fmaf(a, b.z, acc.z);
-      acc.w = fmaf(a, b.w, acc.w);
-    };
-    if (d.band_val) {
-      // consecutive columns: the row's first column, then its values alone
-      // (4 bytes per entry), in stored order
-      if (s < e) {
-        const float4 *sp = st4 + (__ldg(d.cv + s).x - w.lo) * TK + tk;
-        const auto addv = [&](float a, const float4 b) {
-          acc.x = fmaf(a, b.x, acc.x);
-          acc.y = fmaf(a, b.y, acc.y);
-          acc.z = fmaf(a, b.z, acc.z);
-          acc.w = fmaf(a, b.w, acc.w);
-        };
-        int32_t q = s;
-        for (; q + 4 <= e; q += 4) {
-          float a[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            a[u] = __ldg(d.band_val + q + u);
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            addv(a[u], sp[(q - s + u) * TK]);
-        }
-        for (; q < e; ++q)
-          addv(__ldg(d.band_val + q), sp[(q - s) * TK]);
-      }
-    } else {
-      int32_t q = s;
-      for (; q + 4 <= e; q += 4) {
-        int2 t[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          t[u] = __ldg(d.cv + q + u);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          add(t[u]);
-      }
-      for (; q < e; ++q)
-        add(__ldg(d.cv + q));
-    }
+  // alpha * sum + beta * C of one row's 4 columns
+  const auto store = [&](int32_t row, const float4 &acc) {
     float *crow = d.C + (int64_t)row * d.ldc + kk;
     const float sum[4] = {acc.x, acc.y, acc.z, acc.w};
     if (vec) {
@@ -290,6 +319,117 @@ __device__ __forceinline__ void staged_item(const SItem &w, const InstDesc &d,
           crow[v] = o;
         }
     }
+  };
+  if (d.band_blk) {
+    // 4 rows per thread: a column's 4 values in one load and its staged row of
+    // B in one, for 16 products; the columns of a row in ascending order. Bound
+    // by the L1 data pipe: a row at a time, each of a warp's 4 to 32 rows read
+    // its values from another line. Blocks of 4 rows read a quarter as often,
+    // and side by side in the order the warp takes them a load is one stretch
+    // of memory. Measured on the 43 banded instances of a 128-instance batch:
+    // row by row 286 us, blocks of 4 226 us, with the row groups' stage reads
+    // in different banks 223 us, with the blocks side by side 195 us (k <= 4:
+    // 82 -> 54 us, 5 to 16: 96 -> 59 us, above: 166 -> 125 us).
+    const auto fma4 = [](float4 &acc, float a, const float4 &b) {
+      acc.x = fmaf(a, b.x, acc.x);
+      acc.y = fmaf(a, b.y, acc.y);
+      acc.z = fmaf(a, b.z, acc.z);
+      acc.w = fmaf(a, b.w, acc.w);
+    };
+    for (int32_t blk = w.row0 / 4 + warp * per + rs; 4 * blk < w.row1; blk += warps * per) {
+      const BandBlock bb = band_block(d.band_rng, d.m, blk);
+      const int P = d.band_p;
+      const float4 *vp = d.band_blk + (int64_t)(blk / P) * d.band_w * P + blk % P;
+      const float4 *sp = st4 + (bb.lo - w.lo) * S + tk;
+      float4 acc[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int c = bb.lo; c <= bb.hi; c += 4, vp += 4 * P, sp += 4 * S) {
+        float4 a[4];  // band_w is a multiple of 4: inside the block's float4s
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          a[u] = __ldg(vp + u * P);
+        if (c >= bb.lo_all && c + 3 <= bb.hi_all) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float4 b = sp[u * S];
+            fma4(acc[0], a[u].x, b);
+            fma4(acc[1], a[u].y, b);
+            fma4(acc[2], a[u].z, b);
+            fma4(acc[3], a[u].w, b);
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (c + u > bb.hi)
+              break;
+            const float4 b = sp[u * S];
+            const float av[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (c + u >= bb.row[i].x && c + u <= bb.row[i].y)
+                fma4(acc[i], av[i], b);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (4 * blk + i < w.row1)
+          store(4 * blk + i, acc[i]);
+    }
+    return;
+  }
+  for (int32_t row = w.row0 + warp * per + rs; row < w.row1; row += warps * per) {
+    const int32_t s = __ldg(d.rp + row), e = __ldg(d.rp + row + 1);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const auto add = [&](int2 t) {
+      const float4 b = st4[(t.x - w.lo) * S + tk];
+      const float a = __int_as_float(t.y);
+      acc.x = fmaf(a, b.x, acc.x);
+      acc.y = fmaf(a, b.y, acc.y);
+      acc.z = fmaf(a, b.z, acc.z);
+      acc.w = fmaf(a, b.w, acc.w);
+    };
+    if (d.band_val) {
+      // consecutive columns: the row's first column, then its values alone
+      // (4 bytes per entry), in stored order
+      if (s < e) {
+        const float4 *sp = st4 + (__ldg(d.cv + s).x - w.lo) * S + tk;
+        const auto addv = [&](float a, const float4 b) {
+          acc.x = fmaf(a, b.x, acc.x);
+          acc.y = fmaf(a, b.y, acc.y);
+          acc.z = fmaf(a, b.z, acc.z);
+          acc.w = fmaf(a, b.w, acc.w);
+        };
+        int32_t q = s;
+        for (; q + 4 <= e; q += 4) {
+          float a[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            a[u] = __ldg(d.band_val + q + u);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            addv(a[u], sp[(q - s + u) * S]);
+        }
+        for (; q < e; ++q)
+          addv(__ldg(d.band_val + q), sp[(q - s) * S]);
+      }
+    } else {
+      int32_t q = s;
+      for (; q + 4 <= e; q += 4) {
+        int2 t[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          t[u] = __ldg(d.cv + q + u);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          add(t[u]);
+      }
+      for (; q < e; ++q)
+        add(__ldg(d.cv + q));
+    }
+    store(row, acc);
   }
 }
 
@@ -338,8 +478,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4)  // 64 registers: 4 blocks p
       else
         batch_bsr_rows<2>(d, w, lane, alpha, beta, beta_nz);
     } else {
-      const PackedRows A{d.rp, d.cv};
-      batch_rows<PackedRows, OFF32>(A, d, w, lane, alpha, beta, beta_nz, pol);
+      batch_rows<OFF32>(d, w, lane, alpha, beta, beta_nz, pol);
     }
     it = __shfl_sync(0xffffffffu, next, 0);
   }
@@ -390,6 +529,43 @@ __global__ void k_rows_consecutive(int32_t m, const int32_t *__restrict__ rp,
       atomicAnd(flag, 0);
       return;
     }
+}
+
+// Every row's first and last column (0, -1 for an empty row) of an instance
+// whose rows' columns are consecutive.
+__global__ void k_band_ranges(int32_t m, const int32_t *__restrict__ rp,
+                              const int32_t *__restrict__ col, int2 *__restrict__ rng) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= m)
+    return;
+  const int32_t s = rp[r], e = rp[r + 1];
+  rng[r] = s < e ? make_int2(col[s], col[s] + (e - s) - 1) : make_int2(0, -1);
+}
+
+// The widest block of 4 rows.
+__global__ void k_band_width(int32_t m, const int2 *__restrict__ rng, int *__restrict__ width) {
+  const int32_t blk = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+  int w = 0;
+  if (4 * (int64_t)blk < m) {
+    const BandBlock b = band_block(rng, m, blk);
+    w = b.hi >= 0 ? b.hi - b.lo + 1 : 0;
+  }
+  w = __reduce_max_sync(0xffffffffu, w);
+  if ((threadIdx.x & 31) == 0 && w > 0)
+    atomicMax(width, w);
+}
+
+__global__ void k_band_fill(int32_t m, const int32_t *__restrict__ rp,
+                            const float *__restrict__ val, const int2 *__restrict__ rng,
+                            int32_t w, int32_t P, float *__restrict__ out) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= m)
+    return;
+  const int32_t blk = (int32_t)(r / 4);
+  const BandBlock b = band_block(rng, m, blk);
+  float *o = out + (((int64_t)(blk / P) * w + (rng[r].x - b.lo)) * P + blk % P) * 4 + r % 4;
+  for (int32_t p = rp[r]; p < rp[r + 1]; ++p, o += 4 * P)
+    *o = val[p];
 }
 
 // The blocks of a BSR instance, column-major (element (i, j) of block p at
@@ -462,6 +638,7 @@ struct perflibs_b200_batch_s {
   pls::DevBuf scalar_rp;  // row pointers of the BSR instances' scalar rows
   pls::DevBuf bsr_cm;     // column-major copies of the blocks read as blocks (path 3)
   pls::DevBuf band_vals;  // the values of the band instances (consecutive columns)
+  pls::DevBuf band_blks, band_rngs;  // the same by blocks of 4 rows, and the rows' ranges
   pls::DevBuf sitems;     // staged items, largest first
   // Per instance, the row ranges left to the per-warp items when staged
   // items are on (the blocks that were not staged).
@@ -549,9 +726,10 @@ void build_staged(Batch *B) {
       to_warps(0, d.m);
       continue;
     }
-    const int32_t ksp0 = 4 * (int32_t)div_up(std::min(d.k, kStageCols), 4);
-    const int32_t wmax = kStageFloats / ksp0;
-    const int32_t rs = wmax / 2;
+    const int32_t tk0 = stage_lanes(d.k);
+    const int32_t wmax = kStageFloats / (4 * stage_stride(tk0));
+    // whole blocks of 4 rows for every lane group of a warp
+    const int32_t rs = wmax / 2 / (4 * (32 / tk0)) * (4 * (32 / tk0));
     const int64_t nblk = div_up((int64_t)d.m, (int64_t)rs);
     win.reserve(sizeof(int4) * nblk);
     k_block_window<<<(unsigned)nblk, 256, 0, B->stream>>>(d.m, rs, d.rp, d.cv, win.as<int4>());
@@ -782,24 +960,74 @@ perflibs_status_t perflibs_b200_batch_create(perflibs_b200_batch_t *out, int32_t
       PLS_CUDA(cudaMemcpyAsync(hf.data(), flags.p, sizeof(int) * count, cudaMemcpyDeviceToHost,
                                B->stream));
       PLS_CUDA(cudaStreamSynchronize(B->stream));
-      int64_t nb = 0;
+      const auto is_band = [&](int32_t i) {
+        return !B->host[i].is_bsr && hf[i] && B->host[i].m > 0 && mats[i]->csr.nnz > 0;
+      };
+      int64_t rows = 0;
       for (int32_t i = 0; i < count; ++i)
-        if (!B->host[i].is_bsr && hf[i])
-          nb += mats[i]->csr.nnz;
+        rows += is_band(i) ? B->host[i].m : 0;
+      B->band_rngs.reserve(sizeof(int2) * std::max<int64_t>(rows, 1));
+      PLS_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * count, B->stream));
+      rows = 0;
+      for (int32_t i = 0; i < count; ++i) {
+        InstDesc &d = B->host[i];
+        if (!is_band(i))
+          continue;
+        int2 *rng = B->band_rngs.as<int2>() + rows;
+        k_band_ranges<<<(unsigned)div_up(d.m, 256), 256, 0, B->stream>>>(d.m, d.rp, d.col, rng);
+        k_band_width<<<(unsigned)div_up(d.m, 4 * 256), 256, 0, B->stream>>>(
+            d.m, rng, flags.as<int>() + i);
+        d.band_rng = rng;
+        d.band_p = 32 / stage_lanes(d.k);
+        rows += d.m;
+      }
+      PLS_LAUNCH_CHECK();
+      std::vector<int> width((size_t)count, 0);
+      PLS_CUDA(cudaMemcpyAsync(width.data(), flags.p, sizeof(int) * count,
+                               cudaMemcpyDeviceToHost, B->stream));
+      PLS_CUDA(cudaStreamSynchronize(B->stream));
+      // By blocks of 4 rows where that takes at most twice the values' memory
+      // (rows of 5 entries, one column further each: 1.6 times), else in
+      // stored order.
+      const auto slots = [&](int32_t i) {
+        return div_up(div_up(B->host[i].m, 4), B->host[i].band_p) * B->host[i].band_p *
+               (div_up(width[i], 4) * 4) * 4;
+      };
+      int64_t nb = 0, nk = 0;
+      for (int32_t i = 0; i < count; ++i)
+        if (is_band(i)) {
+          if (slots(i) <= 2 * mats[i]->csr.nnz)
+            nk += slots(i);
+          else
+            nb += mats[i]->csr.nnz;
+        }
       B->band_vals.reserve(sizeof(float) * std::max<int64_t>(nb, 1));
-      nb = 0;
+      B->band_blks.reserve(sizeof(float) * std::max<int64_t>(nk, 1));
+      PLS_CUDA(cudaMemsetAsync(B->band_blks.p, 0, sizeof(float) * nk, B->stream));
+      nb = nk = 0;
       for (int32_t i = 0; i < count; ++i) {
         InstDesc &d = B->host[i];
         d.band_val = nullptr;
-        if (d.is_bsr || !hf[i])
+        d.band_blk = nullptr;
+        if (!is_band(i))
           continue;
         const int64_t nnz = mats[i]->csr.nnz;
-        float *out = B->band_vals.as<float>() + nb;
-        if (nnz > 0)
+        if (slots(i) <= 2 * nnz) {
+          float *out = B->band_blks.as<float>() + nk;
+          d.band_w = (int32_t)div_up(width[i], 4) * 4;
+          k_band_fill<<<(unsigned)div_up(d.m, 256), 256, 0, B->stream>>>(d.m, d.rp, d.val,
+                                                                          d.band_rng, d.band_w,
+                                                                          d.band_p, out);
+          PLS_LAUNCH_CHECK();
+          d.band_blk = reinterpret_cast<const float4 *>(out);
+          nk += slots(i);
+        } else {
+          float *out = B->band_vals.as<float>() + nb;
           PLS_CUDA(cudaMemcpyAsync(out, d.val, sizeof(float) * nnz, cudaMemcpyDeviceToDevice,
                                    B->stream));
-        d.band_val = out;
-        nb += nnz;
+          d.band_val = out;
+          nb += nnz;
+        }
       }
       PLS_CUDA(cudaStreamSynchronize(B->stream));
     }

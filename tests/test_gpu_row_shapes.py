@@ -312,3 +312,59 @@ def test_diagonal_form_beyond_32_bit_offsets():
     B64 = B[:, :k].double().cpu().numpy()
     v64 = v.astype(np.float32).astype(np.float64)
     check(C.cpu().numpy(), oracle.csr_spmm(rp, c, v64, B64, k), oracle.csr_spmm(rp, c, np.abs(v64), np.abs(B64), k), 1e-6)
+
+
+# ------------------------------------------------------------------- batch
+
+
+def skyline(n, lo_of, len_of):
+    """Rows of consecutive columns: row r holds columns lo_of(r) .. + len_of(r)."""
+    r = np.arange(n)
+    lo = np.clip(lo_of(r), 0, n - 1)
+    lens = np.clip(len_of(r), 0, n - lo)
+    rp = np.zeros(n + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    col = np.repeat(lo, lens) + np.arange(rp[-1]) - np.repeat(rp[:-1], lens)
+    return rp, col.astype(np.int32)
+
+
+@pytest.mark.parametrize("k", [1, 3, 4, 9, 13, 32, 47])
+def test_batch_band_rows_by_blocks_of_four(k):
+    """Rows of consecutive columns whose blocks of 4 overlap fully, partly or
+    not at all (those keep the stored order), with empty rows, a row count
+    that is no multiple of 4 and one row alone, staged and not, with beta."""
+    import torch
+
+    rng = np.random.default_rng(k)
+    shapes = [(1, lambda r: r, lambda r: 1 + 0 * r),
+              (1023, lambda r: r - 2, lambda r: 5 + 0 * r),
+              (1301, lambda r: r - 40, lambda r: 81 + 0 * r),
+              (770, lambda r: r - r % 7, lambda r: 3 + r % 11),
+              (901, lambda r: r - 20, lambda r: np.where(r % 5 == 0, 0, 40)),
+              (640, lambda r: (r * 37) % 600, lambda r: 8 + 0 * r)]
+    mats, Bs, Cs, C0s, refs = [], [], [], [], []
+    for n, lo_of, len_of in shapes:
+        rp, c = skyline(n, lo_of, len_of)
+        v = rng.uniform(-1, 1, len(c)).astype(np.float32)
+        B = rng.uniform(-1, 1, (n, k)).astype(np.float32)
+        C0 = rng.uniform(-1, 1, (n, k)).astype(np.float32)
+        v64, B64 = v.astype(np.float64), B.astype(np.float64)
+        ab, s = oracle.csr_spmm(rp, c, v64, B64, k), oracle.csr_spmm(rp, c, np.abs(v64), np.abs(B64), k)
+        refs.append((0.5 * ab - 2.0 * C0, 0.5 * s + 2 * np.abs(C0)))
+        mats.append(pls.SpMat.csr(n, n, rp, c, v))
+        Bs.append(torch.tensor(B, device="cuda"))
+        Cs.append(torch.tensor(C0, device="cuda"))
+        C0s.append(torch.tensor(C0, device="cuda"))
+    ks = [k] * len(mats)
+    torch.cuda.synchronize()
+    bt = pls.Batch(mats, ks, [b.data_ptr() for b in Bs], ks, [c.data_ptr() for c in Cs], ks)
+    assert bt.stage_info()["staged_items"] > 0
+    for staging in (True, False):
+        bt.set_staging(staging)
+        for C, C0 in zip(Cs, C0s):
+            C.copy_(C0)
+        torch.cuda.synchronize()
+        bt.exec(0.5, -2.0)
+        torch.cuda.synchronize()
+        for C, (ref, scale) in zip(Cs, refs):
+            check(C.cpu().numpy(), ref, scale, 1e-5)

@@ -530,29 +530,45 @@ template <class X> bool matches(const Mat *A) {
 // call took 1.56 ms as one launch, 1.35 ms in 4 bands, 1.32 ms in 8 and
 // 1.53 ms in 16: smaller bands add more launch and copy overhead than they
 // hide.
+//
+// Where the first rows read only the first part of x (stencils, bands), x comes
+// in piece by piece, each band waiting for the columns that it reads, so x's
+// copy runs beside y's in the other direction; smaller bands then start y's
+// copy earlier. A 5-point Laplacian of 1000^2 (8 MB each way, pinned), 2 bands
+// behind x's copy -> 7 bands with x in pieces: 331 -> 302 us; on a host whose
+// uploads ran at 19 GB/s 551 -> 320 us.
 constexpr int64_t kBandBytes = 4 << 20;
+constexpr int64_t kLocalBandBytes = 1 << 20;
 constexpr int kMaxBands = 8;
 constexpr int kMaxHostBands = 64;  // bound of an explicit band count
 
 template <class X>
-int band_count(const Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen) {
+int band_count(Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen, cudaStream_t s) {
   if (trans != PERFLIBS_SPARSE_OPERATION_NOTRANS || alpha == X(0) || xlen == 0)
     return 1;
   if (A->fmt != Fmt::SELL && A->fmt != Fmt::CSR)
     return 1;
   if (A->host_bands > 0)
     return A->host_bands;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(kMaxBands, ylen * (int64_t)sizeof(X) / kBandBytes));
+  const int64_t bytes = ylen * (int64_t)sizeof(X);
+  if (bytes < 2 * kLocalBandBytes)
+    return 1;
+  csr_find_reach(A->csr, A->m, A->ybuf.as<int32_t>(), s);  // ybuf is not in use yet
+  const bool local = 2 * csr_reach(A->csr, A->m, A->m / kMaxBands) <= xlen;
+  return (int)std::max<int64_t>(
+      1, std::min<int64_t>(kMaxBands, bytes / (local ? kLocalBandBytes : kBandBytes)));
 }
 
-// The bands' kernels run in band order on the handle's stream; a band's
-// event releases the copy of its rows on the copy stream. All kernels are
-// queued before the first copy: with pageable host memory a copy may block
-// the host, and the kernels are already queued then. (Bands on several
-// streams at once measured slower: the first band then shares the GPU with
-// the others and its copy starts later.)
+// The bands' kernels run in band order on the handle's stream, each after the
+// piece of x (with beta != 0 also its rows of y) that the upload stream brings
+// it; a band's event releases the copy of its rows on the copy stream. With
+// pageable host memory a copy may block the host, so then all kernels are
+// queued before the first copy back. (Bands on several streams at once
+// measured slower: the first band then shares the GPU with the others and its
+// copy starts later.)
 template <class X>
-bool spmv_banded(Mat *A, int n_bands, X alpha, X beta, X *y_host, cudaStream_t s) {
+bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X beta, X *y_host,
+                 cudaStream_t s) {
   const std::vector<RowBand> *bands;
   if (A->fmt == Fmt::SELL) {
     sell_plan_bands(A->sell, A->m, n_bands);
@@ -564,29 +580,70 @@ bool spmv_banded(Mat *A, int n_bands, X alpha, X beta, X *y_host, cudaStream_t s
   const size_t nb = bands->size();
   if (nb < 2)
     return false;
+  csr_find_reach(A->csr, A->m, A->ybuf.as<int32_t>(), s);
   BandLanes &L = A->lanes;
-  const X *xd = A->xbuf.as<X>();
+  X *xd = A->xbuf.as<X>();
   X *yd = A->ybuf.as<X>();
   const int tpr = A->cfg.kind == Kind::CSR_SPLIT ? 0
                   : A->cfg.tpr > 0              ? A->cfg.tpr
                                                 : default_config(A).tpr;
+  // y's rows may go back while x is still read: all of x first when they share
+  // memory.
+  const bool shared = x_host < y_host + A->m && y_host < x_host + xlen;
+  cudaPointerAttributes at{};
+  const bool pinned = cudaPointerGetAttributes(&at, y_host) == cudaSuccess &&
+                      at.type == cudaMemoryTypeHost;
+  cudaStream_t c = L.copy_stream(), u = L.upload_stream();
+  const auto copy_back = [&](size_t i) {
+    const RowBand &b = (*bands)[i];
+    PLS_CUDA(cudaStreamWaitEvent(c, L.event(i), 0));
+    PLS_CUDA(cudaMemcpyAsync(y_host + b.r0, yd + b.r0, sizeof(X) * (size_t)(b.r1 - b.r0),
+                             cudaMemcpyDeviceToHost, c));
+  };
+  // A call that fails on the way returns with none of its copies in flight.
+  struct Drain {
+    cudaStream_t st[3];
+    ~Drain() {
+      for (cudaStream_t q : st)
+        if (q)
+          cudaStreamSynchronize(q);
+    }
+  } drain{{u, s, c}};
+  // Events [0, nb): a band's kernels done; nb: work queued on the handle's
+  // stream before this call; nb + 1 + i: band i's upload done.
+  PLS_CUDA(cudaEventRecord(L.event(nb), s));
+  PLS_CUDA(cudaStreamWaitEvent(u, L.event(nb), 0));
+  int64_t have = 0;  // elements of x uploaded
   for (size_t i = 0; i < nb; ++i) {
     const RowBand &b = (*bands)[i];
+    const int64_t need = shared ? xlen : csr_reach(A->csr, A->m, b.r1);
+    if (need > have)
+      PLS_CUDA(cudaMemcpyAsync(xd + have, x_host + have, sizeof(X) * (size_t)(need - have),
+                               cudaMemcpyHostToDevice, u));
+    // With beta = 0 every kernel writes all of y without reading it (the
+    // reference's y = alpha*A*x: old values, NaN included, do not propagate).
+    if (beta != X(0))
+      PLS_CUDA(cudaMemcpyAsync(yd + b.r0, y_host + b.r0, sizeof(X) * (size_t)(b.r1 - b.r0),
+                               cudaMemcpyHostToDevice, u));
+    if (need > have || beta != X(0)) {
+      PLS_CUDA(cudaEventRecord(L.event(nb + 1 + i), u));
+      PLS_CUDA(cudaStreamWaitEvent(s, L.event(nb + 1 + i), 0));
+    }
+    have = std::max(have, need);
     if (A->fmt == Fmt::SELL)
       spmv_sell_band<X>(A->sell, b, xd, yd, alpha, beta, s);
     else
       spmv_csr_band<X>(A->csr, b, tpr, xd, yd, alpha, beta, s);
     PLS_CUDA(cudaEventRecord(L.event(i), s));
+    if (pinned)
+      copy_back(i);
   }
-  cudaStream_t c = L.copy_stream();
-  for (size_t i = 0; i < nb; ++i) {
-    const RowBand &b = (*bands)[i];
-    PLS_CUDA(cudaStreamWaitEvent(c, L.event(i), 0));
-    PLS_CUDA(cudaMemcpyAsync(y_host + b.r0, yd + b.r0, sizeof(X) * (size_t)(b.r1 - b.r0),
-                             cudaMemcpyDeviceToHost, c));
-  }
-  // The copy stream waited for the last band, so once it is idle so is `s`.
+  for (size_t i = 0; i < nb && !pinned; ++i)
+    copy_back(i);
+  // The copy stream waited for the last band, so once it is idle so are `s`
+  // and the upload stream.
   PLS_CUDA(cudaStreamSynchronize(c));
+  drain = Drain{};
   A->last_host_bands = (int)nb;
   return true;
 }
@@ -611,16 +668,14 @@ perflibs_status_t spmv_exec_host(int trans, X alpha, Mat *A, const X *x, X beta,
     if (ylen == 0)
       return PERFLIBS_STATUS_SUCCESS;
     A->xbuf.reserve(sizeof(X) * std::max<int64_t>(xlen, 1));
-    A->ybuf.reserve(sizeof(X) * ylen);
+    A->ybuf.reserve(std::max<size_t>(sizeof(X) * ylen, sizeof(int32_t) * kReachParts));
+    const int n_bands = band_count<X>(A, trans, alpha, xlen, ylen, s);
+    if (n_bands > 1 && spmv_banded<X>(A, n_bands, alpha, x, xlen, beta, y, s))
+      return PERFLIBS_STATUS_SUCCESS;
     if (xlen > 0)
       PLS_CUDA(cudaMemcpyAsync(A->xbuf.p, x, sizeof(X) * xlen, cudaMemcpyHostToDevice, s));
-    // With beta = 0 every kernel writes all of y without reading it (the
-    // reference's y = alpha*A*x: old values, NaN included, do not propagate).
     if (beta != X(0))
       PLS_CUDA(cudaMemcpyAsync(A->ybuf.p, y, sizeof(X) * ylen, cudaMemcpyHostToDevice, s));
-    const int n_bands = band_count<X>(A, trans, alpha, xlen, ylen);
-    if (n_bands > 1 && spmv_banded<X>(A, n_bands, alpha, beta, y, s))
-      return PERFLIBS_STATUS_SUCCESS;
     const perflibs_status_t st =
         spmv_device<X>(trans, alpha, A, A->xbuf.as<X>(), beta, A->ybuf.as<X>(), s);
     PLS_CUDA(cudaMemcpyAsync(y, A->ybuf.p, sizeof(X) * ylen, cudaMemcpyDeviceToHost, s));

@@ -234,12 +234,13 @@ struct BandPlan {
   }
 };
 
-// The copy stream and events of banded host-buffer calls, created on first
-// use on the handle's GPU: event i marks the end of band i's kernels on the
-// handle's stream, and the copy stream waits for it before copying the
-// band's rows of y to the host.
+// The copy streams and events of banded host-buffer calls, created on first
+// use on the handle's GPU: the upload stream brings x (and y) in, piece by
+// piece, and the handle's stream waits for the piece a band needs; event i
+// marks the end of band i's kernels on the handle's stream, and the copy
+// stream waits for it before copying the band's rows of y to the host.
 struct BandLanes {
-  cudaStream_t copy = nullptr;
+  cudaStream_t copy = nullptr, upload = nullptr;
   std::vector<cudaEvent_t> ev;
   BandLanes() = default;
   BandLanes(const BandLanes &) = delete;
@@ -249,6 +250,13 @@ struct BandLanes {
       cudaEventDestroy(e);
     if (copy)
       cudaStreamDestroy(copy);
+    if (upload)
+      cudaStreamDestroy(upload);
+  }
+  cudaStream_t upload_stream() {
+    if (!upload)
+      PLS_CUDA(cudaStreamCreateWithFlags(&upload, cudaStreamNonBlocking));
+    return upload;
   }
   cudaStream_t copy_stream() {
     if (!copy)
@@ -379,6 +387,9 @@ struct CsrDev {
   uint64_t vals_version = 0;  // counts value updates (invalidates value copies)
   int32_t ncols = 0;  // columns (bound of col); 0 when not recorded
   int32_t max_row = INT32_MAX;  // longest row; INT32_MAX when not recorded
+  // One past the last column that the rows of each of kReachParts equal parts
+  // read, or any row before them (found on the first banded host-buffer call).
+  std::vector<int32_t> reach;
   Vt vt = Vt::F64;
   // Reduced-precision copy of the values used by the kernels when the
   // handle's storage mode asks for one.
@@ -593,6 +604,11 @@ void csr_plan_bands(CsrDev &c, int32_t m, int n_bands);
 template <class X>
 void spmv_sell_band(const SellDev &s, const RowBand &b, const X *x, X *y, X alpha, X beta,
                     cudaStream_t st);
+// CsrDev::reach (`scratch`: kReachParts device words), and the columns
+// [0, result) that rows [0, r1) read.
+constexpr int kReachParts = 64;
+void csr_find_reach(CsrDev &c, int32_t m, int32_t *scratch, cudaStream_t s);
+int64_t csr_reach(const CsrDev &c, int32_t m, int64_t r1);
 // tpr = 0 runs the long-row split kernels (threshold c.long_threshold).
 template <class X>
 void spmv_csr_band(const CsrDev &c, const RowBand &b, int tpr, const X *x, X *y, X alpha,

@@ -368,3 +368,61 @@ def test_batch_band_rows_by_blocks_of_four(k):
         torch.cuda.synchronize()
         for C, (ref, scale) in zip(Cs, refs):
             check(C.cpu().numpy(), ref, scale, 1e-5)
+
+
+# ------------------------------------------- host-buffer calls, x in pieces
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("kind", ["laplace", "empty_start", "reversed", "wide"])
+def test_host_exec_uploads_x_as_the_bands_need_it(kind, dtype):
+    """Local rows (x comes in pieces), rows of which the first read nothing or
+    the last part of x, more columns than rows; CSR and SELL; pinned and
+    pageable vectors, x and y in the same array, asked-for band counts, other
+    x on the next call."""
+    import torch
+
+    rng = np.random.default_rng(3)
+    m = 700_001
+    n = m if kind != "wide" else 900_007
+    r = np.arange(m)
+    if kind == "laplace":
+        cols = np.clip(r[:, None] + np.array([-900, -1, 0, 1, 900]), 0, n - 1)
+    elif kind == "wide":
+        cols = np.clip((r * 9 // 7)[:, None] + np.array([0, 3, 40]), 0, n - 1)
+    else:
+        cols = np.stack([n - 1 - r, np.maximum(n - 5 - r, 0)], 1) if kind == "reversed" else r[:, None]
+    cols = np.sort(cols, 1)
+    keep = np.ones(cols.shape, bool)
+    keep[:, 1:] = cols[:, 1:] != cols[:, :-1]
+    if kind == "empty_start":
+        keep[: m // 3] = False
+    rp = np.zeros(m + 1, np.int32)
+    rp[1:] = np.cumsum(keep.sum(1))
+    c = cols[keep].astype(np.int32)
+    v = rng.uniform(-1, 1, len(c)).astype(dtype)
+    tol = 1e-12 if dtype == np.float64 else 1e-5
+    y0 = W.uniform_vector(m, 5).astype(dtype)
+    for cfg in ((pls.KIND_CSR, 0, 0, 2), (pls.KIND_SELL, 32, 256, 0)):
+        A = pls.SpMat.csr(m, n, rp, c, v)
+        assert A.force_config(*cfg) == 0
+        assert A.optimize() == 0
+        for bands, seed in ((0, 1), (3, 2), (64, 3), (0, 4)):
+            A.set_host_bands(bands)
+            x = W.uniform_vector(n, seed).astype(dtype)
+            ref = oracle.csr_spmv(rp, c, v.astype(np.float64), x.astype(np.float64),
+                                  y=y0.astype(np.float64), alpha=1.5, beta=-0.5)
+            scale = 1.5 * oracle.csr_absdot(rp, c, v.astype(np.float64), x.astype(np.float64)) \
+                + 0.5 * np.abs(y0.astype(np.float64))
+            check(A.spmv(x, y0.copy(), alpha=1.5, beta=-0.5), ref, scale, tol)
+            if bands:
+                assert A.host_bands_used() > 1
+            xp = torch.tensor(x).pin_memory().numpy()
+            yp = torch.tensor(y0).pin_memory().numpy()
+            check(A.spmv(xp, yp, alpha=1.5, beta=-0.5), ref, scale, tol)
+            ref1 = oracle.csr_spmv(rp, c, v.astype(np.float64), x.astype(np.float64))
+            yp[:] = np.nan
+            check(A.spmv(xp, yp), ref1, scale, tol)
+            if m == n:
+                check(A.spmv(xp, xp), ref1, scale, tol)
+        A.destroy()

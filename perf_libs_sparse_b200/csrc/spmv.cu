@@ -56,7 +56,7 @@ __device__ __forceinline__ Acc csr_lane_sum(uint32_t j, uint32_t e, const int32_
     Acc xv[G];
 #pragma unroll
     for (int u = 0; u < G; ++u)
-      xv[u] = j + u * STEP < e ? to_acc<Acc>(ld_keep(x + c[u], pol.keep)) : Acc(0);
+      xv[u] = j + u * STEP < e ? to_acc<Acc>(ld_gather(x + c[u], pol.keep)) : Acc(0);
 #pragma unroll
     for (int u = 0; u < G; ++u)
       if (j + u * STEP < e)
@@ -80,10 +80,10 @@ template <int TPR, bool LONG, class V, class X>
 __global__ void __launch_bounds__(256)
     k_csr_vector(int32_t m, const int32_t *__restrict__ rp,
                  const int32_t *__restrict__ col, const V *__restrict__ val,
-                 const X *__restrict__ x, X *__restrict__ y, X alpha, X beta,
-                 int beta_nz, int32_t skip_len) {
+                 const X *xg, X *y, X alpha, X beta, int beta_nz, int32_t skip_len) {
   using Acc = typename AccOf<V, X>::type;
   constexpr int G = csr_group(TPR);
+  chain_next();
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t row = gid / TPR;
   const int sub = threadIdx.x & (TPR - 1);
@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(256)
     e = __ldg(rp + row + 1);
     live = !(skip_len > 0 && e - s > skip_len);  // uniform across the row's lanes
   }
+  const X *x = chain_wait(xg);
   const L2Policy pol = make_l2_policy();
   const bool big = LONG && live && e - s > csr_long_len(TPR);
   Acc sum = 0;
@@ -157,9 +158,9 @@ static void launch_csr_vector(const CsrDev &c, int64_t r0, int32_t m, const X *x
   if constexpr (TPR < 32)
     if (has_long)
       kern = k_csr_vector<TPR, true, V, X>;
-  kern<<<(unsigned)blocks, 256, 0, s>>>(
-      m, c.row_ptr.as<int32_t>() + r0, c.col.as<int32_t>(), (const V *)c.ev(), x, y + r0,
-      alpha, beta, beta != X(0), skip);
+  PLS_CUDA(launch_chained(kern, (unsigned)blocks, 256, s, m, c.row_ptr.as<int32_t>() + r0,
+                          c.col.as<int32_t>(), (const V *)c.ev(), x, y + r0, alpha, beta,
+                          beta != X(0), skip));
 }
 
 template <class V, class X>
@@ -270,7 +271,7 @@ __device__ __forceinline__ typename AccOf<V, X>::type sell_row_sum(const V *vp, 
     Acc xv[kSellGroup];
 #pragma unroll
     for (int u = 0; u < kSellGroup; ++u)
-      xv[u] = j + u < len ? to_acc<Acc>(ld_keep(xb + o[u], pol.keep)) : Acc(0);
+      xv[u] = j + u < len ? to_acc<Acc>(ld_gather(xb + o[u], pol.keep)) : Acc(0);
 #pragma unroll
     for (int u = 0; u < kSellGroup; ++u)
       if (j + u < len)
@@ -298,6 +299,12 @@ __device__ __forceinline__ typename AccOf<V, X>::type sell_row_sum(const V *vp, 
 // and the finisher fences before it reads them through L2, the pattern of
 // the CUDA programming guide's last-block reduction. The finisher puts the
 // count back to zero, so done[] is all zero between launches.
+//
+// Launched chained (launch_chained), with chain_next only after a thread's
+// sum: CTAs of the next product that start while many of this one run land
+// unevenly on the SMs, the widest chunks on few of them. Ordinary launch /
+// chain_next first / after the sum, us: random 100,003 x 12 11.9 / 13.5 / 9.0,
+// power-law 200,003 39.8 / 48.4 / 37.5, Laplacian 512^2 7.9 / 5.6 / 5.5.
 template <int C, class V, class O, class X>
 __global__ void __launch_bounds__(kSellThreads, kSellBlocksPerSm)
     k_sell(int64_t nC, int64_t c_base, int32_t split_w, int32_t slice_w, int64_t n_items,
@@ -305,10 +312,11 @@ __global__ void __launch_bounds__(kSellThreads, kSellBlocksPerSm)
            const int32_t *__restrict__ order, const int64_t *__restrict__ cs,
            const int32_t *__restrict__ cl, const int32_t *__restrict__ cmin,
            const int32_t *__restrict__ perm, const V *__restrict__ vals,
-           const O *__restrict__ offs, const X *__restrict__ x, X *__restrict__ y,
+           const O *__restrict__ offs, const X *xg, X *y,
            typename AccOf<V, X>::type *__restrict__ part, int32_t *__restrict__ done, X alpha,
            X beta, int beta_nz) {
   using Acc = typename AccOf<V, X>::type;
+  const X *x = chain_wait(xg);
   const L2Policy pol = make_l2_policy();
   if (blockIdx.x < slice_blocks) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,6 +331,7 @@ __global__ void __launch_bounds__(kSellThreads, kSellBlocksPerSm)
       const X *xb = x + __ldg(cmin + w.x);
       v = sell_row_sum<C, V, O, X>(vals + base, offs + base, xb, w.z - w.y, pol);
     }
+    chain_next();
     // The item is read again rather than kept in registers over the sum.
     const int4 w = __ldg(items + it);
     const int lane = threadIdx.x & 31;
@@ -364,6 +373,7 @@ __global__ void __launch_bounds__(kSellThreads, kSellBlocksPerSm)
   const int32_t dst = __ldg(perm + c * C + r);
   const X *xb = x + (w > 0 ? cm : 0);
   const Acc acc = sell_row_sum<C, V, O, X>(vals + base, offs + base, xb, w, pol);
+  chain_next();
   if (dst >= 0)
     store_y(y, dst, acc, alpha, beta, beta_nz);
 }
@@ -407,10 +417,11 @@ static void launch_sell(const SellDev &s, const SellWork &w, const X *x, X *y, X
   const int64_t chunk_blocks = div_up(w.n_chunks * C, kSellThreads);
   if (slice_blocks + chunk_blocks == 0)
     return;
-  k_sell<C, V, O, X><<<(unsigned)(slice_blocks + chunk_blocks), kSellThreads, 0, st>>>(
-      w.n_chunks, w.c_base, w.split_w, w.slice_w, w.n_items, slice_blocks, w.items, w.order,
+  PLS_CUDA(launch_chained(
+      k_sell<C, V, O, X>, (unsigned)(slice_blocks + chunk_blocks), kSellThreads, st, w.n_chunks,
+      w.c_base, w.split_w, w.slice_w, w.n_items, slice_blocks, w.items, w.order,
       s.cs.as<int64_t>(), s.cl.as<int32_t>(), s.col_min.as<int32_t>(), s.permd2in.as<int32_t>(),
-      s.vals.as<V>(), s.offsets.as<O>(), x, y, (Acc *)w.part, w.done, alpha, beta, bnz);
+      s.vals.as<V>(), s.offsets.as<O>(), x, y, (Acc *)w.part, w.done, alpha, beta, bnz));
 }
 
 template <int C, class V, class X>
@@ -880,16 +891,12 @@ void spmv_dense(const DenseDev &d, int32_t m, int32_t n, bool trans,
 
 // ---------------------------------------------------------------- BSR
 
-// K consecutive values at p: whole 16-byte vectors (8 or 4 bytes when K
-// elements are fewer) with VECT (p is then aligned to them), else one by one;
-// STREAM marks whole vectors read once.
-template <int K, bool VECT, bool STREAM, class T>
-__device__ __forceinline__ void ld_consecutive(const T *p, T (&v)[K]) {
-  constexpr int bytes = K * (int)sizeof(T);
-  if constexpr (!VECT || bytes < 4 || K == 1) {
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-      v[i] = __ldg(p + i);
+// W consecutive values at p, aligned to their size: whole 16-byte vectors,
+// read once, or 8, 4 or 2 bytes.
+template <int W, class V> __device__ __forceinline__ void ld_values(const V *p, V (&v)[W]) {
+  constexpr int bytes = W * (int)sizeof(V);
+  if constexpr (W == 1) {
+    v[0] = p[0];
   } else if constexpr (bytes == 4) {
     const unsigned t = __ldg(reinterpret_cast<const unsigned *>(p));
     memcpy(v, &t, 4);
@@ -897,13 +904,9 @@ __device__ __forceinline__ void ld_consecutive(const T *p, T (&v)[K]) {
     const uint2 t = __ldg(reinterpret_cast<const uint2 *>(p));
     memcpy(v, &t, 8);
   } else {
-    static_assert(bytes % 16 == 0, "whole vectors");
-#pragma unroll
-    for (int h = 0; h < bytes / 16; ++h) {
-      const uint4 t = STREAM ? __ldcs(reinterpret_cast<const uint4 *>(p) + h)
-                             : __ldg(reinterpret_cast<const uint4 *>(p) + h);
-      memcpy(reinterpret_cast<char *>(v) + 16 * h, &t, 16);
-    }
+    static_assert(bytes == 16, "one vector");
+    const uint4 t = __ldcs(reinterpret_cast<const uint4 *>(p));
+    memcpy(v, &t, 16);
   }
 }
 
@@ -927,8 +930,8 @@ __device__ __forceinline__ void ld_consecutive(const T *p, T (&v)[K]) {
 template <int BS, bool RM, bool XVEC, class V, class X>
 __global__ void __launch_bounds__(256)
     k_bsr_vec(int32_t mb, int lg_g, const int32_t *__restrict__ rp,
-              const int32_t *__restrict__ col, const V *__restrict__ val,
-              const X *__restrict__ x, X *__restrict__ y, X alpha, X beta, int beta_nz) {
+              const int32_t *__restrict__ col, const V *__restrict__ val, const X *xg, X *y,
+              X alpha, X beta, int beta_nz) {
   using Acc = typename AccOf<V, X>::type;
   constexpr int E = BS * BS;
   constexpr int WV = 16 / (int)sizeof(V);
@@ -937,6 +940,7 @@ __global__ void __launch_bounds__(256)
   constexpr int RUN = W < BS ? W : BS;  // consecutive values on one block line
   constexpr int LINES = W / RUN;        // block lines (rows when RM) per lane
   constexpr int NR = RM ? LINES : RUN, NC = RM ? RUN : LINES;
+  chain_next();
   const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
   const int64_t br = t >> lg_g;
   const int G = 1 << lg_g;
@@ -955,12 +959,22 @@ __global__ void __launch_bounds__(256)
   for (int r = 0; r < NR; ++r)
     acc[r] = Acc(0);
   int32_t next = b < b1 ? __ldg(col + b) : 0;
+  const X *x = chain_wait(xg);
   while (b < b1) {
     const int32_t c = next;
     V a[W];
-    ld_consecutive<W, true, true>(val + (int64_t)b * E + e0, a);
+    ld_values(val + (int64_t)b * E + e0, a);
     X xv[NC];
-    ld_consecutive<NC, XVEC, false>(x + (int64_t)c * BS + j0, xv);
+    if constexpr (XVEC) {
+      ld_gather<NC>(x + (int64_t)c * BS + j0, xv);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        X one[1];
+        ld_gather<1>(x + (int64_t)c * BS + j0 + j, one);
+        xv[j] = one[0];
+      }
+    }
     b += step;
     next = b < b1 ? __ldg(col + b) : 0;
 #pragma unroll
@@ -1044,8 +1058,8 @@ void spmv_bsr(const BsrDev &b, const X *x, X *y, X alpha, X beta,
         const unsigned grid = (unsigned)div_up((int64_t)b.mb << lg_g, 256);
         const bool xvec = (uintptr_t)x % 16 == 0;  // else x is read element by element
         auto kern = xvec ? k_bsr_vec<BS, RM, true, V, X> : k_bsr_vec<BS, RM, false, V, X>;
-        kern<<<grid, 256, 0, s>>>(b.mb, lg_g, b.row_ptr.as<int32_t>(), b.col.as<int32_t>(),
-                                  (const V *)b.ev(), x, y, alpha, beta, bnz);
+        PLS_CUDA(launch_chained(kern, grid, 256, s, b.mb, lg_g, b.row_ptr.as<int32_t>(),
+                                b.col.as<int32_t>(), (const V *)b.ev(), x, y, alpha, beta, bnz));
       };
       const auto by_layout = [&](auto bs_tag) {
         if (b.layout == PERFLIBS_ROW_MAJOR)

@@ -426,3 +426,68 @@ def test_host_exec_uploads_x_as_the_bands_need_it(kind, dtype):
             if m == n:
                 check(A.spmv(xp, xp), ref1, scale, tol)
         A.destroy()
+
+
+# -------------------------------------------------------- chained launches
+
+
+@pytest.mark.parametrize("fmt", ["csr1", "csr4", "csr_long", "sell", "sell_slices", "bsr2", "bsr8"])
+def test_chained_products_read_what_the_product_before_wrote(fmt):
+    """60 products, each on the result of the one before (beta = 0 and in
+    place of the old y), queued at once, with a kernel of another library
+    between some of them, and replayed from a graph: the bits of the same
+    products with a synchronisation after each."""
+    import torch
+
+    rng = np.random.default_rng(6)
+    n = 4096
+    if fmt.startswith("bsr"):
+        bs = int(fmt[3:])
+        rp, c, _ = csr_of_lengths(np.full(n // bs, 3), n // bs, rng)
+        A = pls.SpMat.bsr(pls.ROW_MAJOR, n, n, bs, rp, c, rng.uniform(-1, 1, len(c) * bs * bs) / (2 * bs))
+    else:
+        lens = rng.integers(0, 9, n)
+        if fmt in ("csr_long", "sell_slices"):
+            lens[::1500] = 900
+        rp, c, v = csr_of_lengths(lens, n, rng)
+        A = pls.SpMat.csr(n, n, rp, c, v / 30)
+        cfg = {"csr1": (pls.KIND_CSR, 0, 0, 1), "csr4": (pls.KIND_CSR, 0, 0, 4), "csr_long": (pls.KIND_CSR, 0, 0, 2),
+               "sell": (pls.KIND_SELL, 32, 0, 0), "sell_slices": (pls.KIND_SELL, 16, 0, 0)}[fmt]
+        assert A.force_config(*cfg) == 0
+        assert A.optimize() == 0
+        assert (A.exec_info()["n_split"] > 0) == (fmt == "sell_slices")
+    s = torch.cuda.Stream()
+    x0 = torch.tensor(W.uniform_vector(n, 3), device="cuda")
+    y0 = torch.tensor(W.uniform_vector(n, 4), device="cuda")
+
+    def chain(a, b, sync):
+        for i in range(60):
+            A.spmv_dev(a.data_ptr(), b.data_ptr(), 1.0, 0.5 if i % 3 == 1 else 0.0, stream=s.cuda_stream)
+            if i % 7 == 3:
+                b.add_(0.25)
+            if sync:
+                s.synchronize()
+            a, b = b, a
+        return a, b
+
+    out = []
+    for mode in ("sync", "queued", "graph"):
+        a, b = torch.cat([x0[:1], x0])[1:], y0.clone()  # one off a 16-byte boundary
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            if mode == "graph":
+                g = torch.cuda.CUDAGraph()
+                g.capture_begin(capture_error_mode="thread_local")
+                chain(a, b, False)
+                g.capture_end()
+                a.copy_(x0)
+                b.copy_(y0)
+                g.replay()
+            else:
+                chain(a, b, mode == "sync")
+        torch.cuda.synchronize()
+        out.append((a.cpu().numpy(), b.cpu().numpy()))
+    assert np.isfinite(out[0][0]).all() and np.abs(out[0][0]).max() > 1e-3
+    for got in out[1:]:
+        np.testing.assert_array_equal(got[0], out[0][0])
+        np.testing.assert_array_equal(got[1], out[0][1])

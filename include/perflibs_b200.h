@@ -110,7 +110,7 @@ enum perflibs_b200_kind {
 /* Force a kernel configuration for the next optimize (the role of the
  * reference's internal set_C / set_sigma knobs, src/matrix_state.cpp:
  * 434-457). sigma is in rows: 0 (no sort) or a multiple of C. tpr 0 picks
- * by mean row length. */
+ * by the mean and the longest row length. */
 perflibs_status_t perflibs_b200_spmat_force_config(perflibs_spmat_t A,
                                                    int kind, int C, int sigma,
                                                    int tpr);
@@ -161,7 +161,9 @@ perflibs_status_t perflibs_b200_spmat_set_spmm_path(perflibs_spmat_t A, int32_t 
  * the first band hide under the device-to-host copy. Applies to NOTRANS
  * with CSR or SELL-C-sigma kernels; every row is summed exactly as in one
  * launch. n_bands = 0 (default) splits results of 8 MB and more into bands
- * of at least 4 MB, up to 8; 1 turns banding off; 2..64 asks for that many
+ * of at least 4 MB, up to 8, and where the first eighth of the rows reads at
+ * most half of x, results of 2 MB and more into bands of at least 1 MB, up to
+ * 8; x is then copied in as the bands need it. 1 turns banding off; 2..64 asks for that many
  * (SELL bands are whole sort windows, so there may be fewer). */
 perflibs_status_t perflibs_b200_spmat_set_host_bands(perflibs_spmat_t A, int32_t n_bands);
 

@@ -406,7 +406,8 @@ perflibs_status_t create_bsr(Mat **out, int layout, int32_t m, int32_t n, int32_
     upload_index(b.row_ptr, row_ptr, (int64_t)b.mb + 1, A->index_base, s);
     upload_index(b.col, col, b.nnzb, A->index_base, s);
     upload(b.vals, vals, sizeof(T) * A->nnz, s);
-    const auto bad = check_compressed(b.mb, b.nb, b.nnzb, b.row_ptr.as<int32_t>(), b.col.as<int32_t>(), s);
+    const auto bad = check_compressed(b.mb, b.nb, b.nnzb, b.row_ptr.as<int32_t>(),
+                                      b.col.as<int32_t>(), s, &b.longest);
     if (bad.first >= 0)
       return param_error(A, 6, "row_ptr decreases or leaves [0, nnzb] at block row " + std::to_string(bad.first));
     if (bad.second >= 0)

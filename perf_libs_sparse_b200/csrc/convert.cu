@@ -374,19 +374,20 @@ __global__ void k_longest_row(int32_t m, const int32_t *__restrict__ rp,
     atomicMax(out, len);
 }
 
-// The longest row of a CSR matrix the library made itself.
-void record_longest_row(CsrDev &c, int32_t m, cudaStream_t s) {
-  c.max_row = 0;
-  if (m <= 0 || c.nnz == 0)
-    return;
+// The longest row of row pointers the library made itself.
+int32_t longest_row(const DevBuf &row_ptr, int32_t m, cudaStream_t s) {
+  int32_t longest = 0;
+  if (m <= 0)
+    return longest;
   DevBuf out;
   out.reserve(4);
   PLS_CUDA(cudaMemsetAsync(out.p, 0, 4, s));
-  k_longest_row<<<(unsigned)div_up(m, 256), 256, 0, s>>>(m, c.row_ptr.as<int32_t>(),
+  k_longest_row<<<(unsigned)div_up(m, 256), 256, 0, s>>>(m, row_ptr.as<int32_t>(),
                                                          out.as<int32_t>());
   PLS_LAUNCH_CHECK();
-  PLS_CUDA(cudaMemcpyAsync(&c.max_row, out.p, 4, cudaMemcpyDeviceToHost, s));
+  PLS_CUDA(cudaMemcpyAsync(&longest, out.p, 4, cudaMemcpyDeviceToHost, s));
   PLS_CUDA(cudaStreamSynchronize(s));
+  return longest;
 }
 
 }  // namespace
@@ -443,7 +444,7 @@ void build_csr_transpose(const CsrDev &c, int32_t m, int32_t n, CsrDev &out,
     PLS_LAUNCH_CHECK();
     PLS_CUDA(cudaStreamSynchronize(s));
   }
-  record_longest_row(T, n, s);
+  T.max_row = longest_row(T.row_ptr, T.nnz > 0 ? n : 0, s);
   out = std::move(T);
 }
 
@@ -599,7 +600,7 @@ int64_t coo_to_csr(int32_t m, int32_t n, int64_t nnz, const int32_t *row, const 
     PLS_LAUNCH_CHECK();
   }
   PLS_CUDA(cudaStreamSynchronize(s));
-  record_longest_row(R, m, s);
+  R.max_row = longest_row(R.row_ptr, R.nnz > 0 ? m : 0, s);
   out = std::move(R);
   return -1;
 }
@@ -644,7 +645,7 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
   });
   PLS_LAUNCH_CHECK();
   PLS_CUDA(cudaStreamSynchronize(s));
-  record_longest_row(R, m, s);
+  R.max_row = longest_row(R.row_ptr, R.nnz > 0 ? m : 0, s);
   out = std::move(R);
 }
 
@@ -730,6 +731,7 @@ void csr_to_bsr(const CsrDev &c, int32_t m, int32_t n, int bs, int layout,
                                            B.row_ptr.as<int32_t>(), B.mb + 1, s));
   }
   PLS_LAUNCH_CHECK();
+  B.longest = longest_row(B.row_ptr, B.mb, s);
   PLS_CUDA(cudaStreamSynchronize(s));
   out = std::move(B);
 }

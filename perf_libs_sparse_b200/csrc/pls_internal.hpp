@@ -442,6 +442,7 @@ struct BsrDev {
   int layout = PERFLIBS_ROW_MAJOR;
   int32_t mb = 0, nb = 0;
   int64_t nnzb = 0;
+  int32_t longest = 0;  // blocks of the longest block row
   DevBuf row_ptr, col, vals;
   Vt vt = Vt::F64;
   DevBuf vals_lo;

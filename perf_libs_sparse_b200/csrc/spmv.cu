@@ -910,6 +910,9 @@ template <int W, class V> __device__ __forceinline__ void ld_values(const V *p, 
   }
 }
 
+constexpr int kBsrLongSteps = 16;
+constexpr int bsr_long_len(int sets) { return kBsrLongSteps * sets; }
+
 // Block sizes 1, 2, 4, 8: G = 2^lg_g lanes per block row. A lane owns W
 // consecutive values of every block it takes (one 16-byte load; fewer for
 // blocks below 16 bytes), LPB lanes a whole block, so the G / LPB lane sets of
@@ -927,7 +930,11 @@ template <int W, class V> __device__ __forceinline__ void ld_values(const V *p, 
 // -> this kernel): bs 8, 60,011 x 8 random blocks 83.6 -> 45.3 us (39 us at
 // the copy rate), bs 4, 100,000 x 6 24.8 -> 19.4 us, bs 2, 300,000 x 12
 // 61.8 -> 28.9 us; bs 8 with BF16 values and FP32 x 41.2 -> 16.7 us.
-template <int BS, bool RM, bool XVEC, class V, class X>
+//
+// LONG: block rows of more than kBsrLongSteps steps are taken by the whole
+// warp, one after another, as in k_csr_vector: on its own lanes such a row is a
+// chain that the launch waits for.
+template <int BS, bool RM, bool XVEC, bool LONG, class V, class X>
 __global__ void __launch_bounds__(256)
     k_bsr_vec(int32_t mb, int lg_g, const int32_t *__restrict__ rp,
               const int32_t *__restrict__ col, const V *__restrict__ val, const X *xg, X *y,
@@ -948,23 +955,16 @@ __global__ void __launch_bounds__(256)
   const int e0 = (g % LPB) * W;  // the lane's first value in a block
   const int line = e0 / BS, at = e0 % BS;
   const int i0 = RM ? line : at, j0 = RM ? at : line;
-  const uint32_t step = G / LPB;
-  uint32_t b = 0, b1 = 0;  // unsigned: b + step passes 2^31 without overflow
+  uint32_t s = 0, e = 0;  // unsigned: s + step passes 2^31 without overflow
   if (br < mb) {
-    b = (uint32_t)__ldg(rp + br) + g / LPB;
-    b1 = (uint32_t)__ldg(rp + br + 1);
+    s = (uint32_t)__ldg(rp + br);
+    e = (uint32_t)__ldg(rp + br + 1);
   }
-  Acc acc[NR];
-#pragma unroll
-  for (int r = 0; r < NR; ++r)
-    acc[r] = Acc(0);
-  int32_t next = b < b1 ? __ldg(col + b) : 0;
+  const bool big = LONG && e - s > (uint32_t)bsr_long_len(G / LPB);
+  const uint32_t b0 = s + g / LPB, b1 = big ? s : e;
+  int32_t next = b0 < b1 ? __ldg(col + b0) : 0;
   const X *x = chain_wait(xg);
-  while (b < b1) {
-    const int32_t c = next;
-    V a[W];
-    ld_values(val + (int64_t)b * E + e0, a);
-    X xv[NC];
+  const auto ld_x = [&](int32_t c, X(&xv)[NC]) {
     if constexpr (XVEC) {
       ld_gather<NC>(x + (int64_t)c * BS + j0, xv);
     } else {
@@ -975,29 +975,85 @@ __global__ void __launch_bounds__(256)
         xv[j] = one[0];
       }
     }
-    b += step;
-    next = b < b1 ? __ldg(col + b) : 0;
+  };
+  const auto add_block = [&](const V(&a)[W], const X(&xv)[NC], Acc(&acc)[NR]) {
 #pragma unroll
     for (int r = 0; r < NR; ++r)
 #pragma unroll
       for (int j = 0; j < NC; ++j)
         acc[r] = fma(to_acc<Acc>(a[RM ? r * RUN + j : j * RUN + r]), to_acc<Acc>(xv[j]), acc[r]);
-  }
-  // Add over the lanes that hold the same rows: those of the block's other
-  // columns and of the other lane sets.
+  };
+  // Adds over the lanes of `lanes` that hold the same rows: those of the
+  // block's other columns and of the other lane sets.
+  const auto add_lanes = [&](int lanes, Acc(&acc)[NR]) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const bool rows_differ = o < LPB && (RM ? o * W >= BS : o * W < BS);
-    if (!rows_differ && o < G) {
+    for (int o = 1; o < 32; o <<= 1) {
+      const bool rows_differ = o < LPB && (RM ? o * W >= BS : o * W < BS);
+      if (!rows_differ && o < lanes) {
 #pragma unroll
-      for (int r = 0; r < NR; ++r)
-        acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+        for (int r = 0; r < NR; ++r)
+          acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+      }
     }
+  };
+  Acc acc[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+    acc[r] = Acc(0);
+  for (uint32_t b = b0; b < b1;) {
+    const int32_t c = next;
+    V a[W];
+    ld_values(val + (int64_t)b * E + e0, a);
+    X xv[NC];
+    ld_x(c, xv);
+    b += G / LPB;
+    next = b < b1 ? __ldg(col + b) : 0;
+    add_block(a, xv, acc);
   }
-  if (br < mb && g < LPB && j0 == 0) {
+  add_lanes(G, acc);
+  if (br < mb && !big && g < LPB && j0 == 0) {
 #pragma unroll
     for (int r = 0; r < NR; ++r)
       store_y(y, br * BS + i0 + r, acc[r], alpha, beta, beta_nz);
+  }
+  if constexpr (LONG) {
+    unsigned todo = __ballot_sync(0xffffffffu, big && g == 0);
+    const uint32_t lane = threadIdx.x & 31;
+    while (todo) {
+      const int o = __ffs(todo) - 1;  // the block row's first lane
+      todo &= todo - 1;
+      const uint32_t ls = __shfl_sync(0xffffffffu, s, o), le = __shfl_sync(0xffffffffu, e, o);
+      const int64_t row = __shfl_sync(0xffffffffu, br, o);
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        acc[r] = Acc(0);
+      constexpr int U = BS == 1 ? 8 : 4;  // blocks in flight: nothing else hides the latency
+      constexpr uint32_t sets = 32 / LPB;
+      for (uint32_t b = ls + lane / LPB; b < le; b += U * sets) {
+        int32_t c[U];
+        V a[U][W];
+        X xv[U][NC];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          c[u] = b + u * sets < le ? __ldg(col + b + u * sets) : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (c[u] >= 0) {
+            ld_values(val + (int64_t)(b + u * sets) * E + e0, a[u]);
+            ld_x(c[u], xv[u]);
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (c[u] >= 0)
+            add_block(a[u], xv[u], acc);
+      }
+      add_lanes(32, acc);
+      if (lane < LPB && j0 == 0) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+          store_y(y, row * BS + i0 + r, acc[r], alpha, beta, beta_nz);
+      }
+    }
   }
 }
 
@@ -1057,7 +1113,19 @@ void spmv_bsr(const BsrDev &b, const X *x, X *y, X alpha, X beta,
           ++lg_g;
         const unsigned grid = (unsigned)div_up((int64_t)b.mb << lg_g, 256);
         const bool xvec = (uintptr_t)x % 16 == 0;  // else x is read element by element
-        auto kern = xvec ? k_bsr_vec<BS, RM, true, V, X> : k_bsr_vec<BS, RM, false, V, X>;
+        auto kern =
+            xvec ? k_bsr_vec<BS, RM, true, false, V, X> : k_bsr_vec<BS, RM, false, false, V, X>;
+        // The whole-warp part where a block row needs it and a warp holds more
+        // lane sets than the block row has. 60,000 block rows of 4 blocks, FP64
+        // (us: a warp per block row and one value per lane / this kernel
+        // without / with the part), and one of 20,000 blocks beside them: bs 1
+        // 68 / 1638 / 59, bs 2 407 / 1730 / 289, bs 4 1950 / 2076 / 1128;
+        // every 200th of 300 blocks instead: 13 / 31 / 6.7, 19 / 32 / 9.8,
+        // 51 / 66 / 44. It takes the kernel from 28 to 40 to 70 registers, so
+        // even block rows run without.
+        if constexpr (BS * BS / W < 32)
+          if (lg_g < 5 && b.longest > bsr_long_len((1 << lg_g) / (BS * BS / W)))
+            kern = xvec ? k_bsr_vec<BS, RM, true, true, V, X> : k_bsr_vec<BS, RM, false, true, V, X>;
         PLS_CUDA(launch_chained(kern, grid, 256, s, b.mb, lg_g, b.row_ptr.as<int32_t>(),
                                 b.col.as<int32_t>(), (const V *)b.ev(), x, y, alpha, beta, bnz));
       };

@@ -491,3 +491,94 @@ def test_chained_products_read_what_the_product_before_wrote(fmt):
     for got in out[1:]:
         np.testing.assert_array_equal(got[0], out[0][0])
         np.testing.assert_array_equal(got[1], out[0][1])
+
+
+def us_per_call(run, n=20):
+    """Device time of one call among n on the current stream."""
+    import torch
+
+    s = torch.cuda.current_stream()
+    for _ in range(3):
+        run(s.cuda_stream)
+    best = np.inf
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(s)
+        for _ in range(n):
+            run(s.cuda_stream)
+        b.record(s)
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3 / n)
+    return best
+
+
+def bsr_product(A, m, n, dtype):
+    import torch
+
+    x = torch.zeros(n, dtype=dtype, device="cuda")
+    y = torch.zeros(m, dtype=dtype, device="cuda")
+    torch.cuda.synchronize()
+    return lambda s: A.spmv_dev(x.data_ptr(), y.data_ptr(), stream=s)
+
+
+@pytest.mark.parametrize("bs", [1, 2, 4])
+def test_bsr_long_block_row_beside_short_ones(bs):
+    """A block row of 20,000 blocks beside thousands of 4 runs as it does alone
+    (then it gets a whole warp too), not on the 2 lane sets of its neighbours
+    (8 to 16 times that): within a factor of 2."""
+    import torch
+
+    rng = np.random.default_rng(bs)
+    nb, long = 30_000, 20_000
+    times = []
+    for short in (0, 20_000):
+        lens = np.r_[np.full(short, 4), long]
+        mb = len(lens)
+        rp = np.zeros(mb + 1, np.int32)
+        rp[1:] = np.cumsum(lens)
+        c = rng.integers(0, nb, int(rp[-1])).astype(np.int32)
+        A = pls.SpMat.bsr(pls.ROW_MAJOR, mb * bs, nb * bs, bs, rp, c, rng.uniform(-1, 1, len(c) * bs * bs))
+        times.append(us_per_call(bsr_product(A, mb * bs, nb * bs, torch.float64)))
+    assert times[1] <= 2 * times[0] + 20
+
+
+@pytest.mark.parametrize("bs", [1, 2, 4, 8])
+@pytest.mark.parametrize("layout", [pls.ROW_MAJOR, pls.COL_MAJOR])
+@pytest.mark.parametrize("dtype,storage", [(np.float64, "native"), (np.float64, "bf16"), (np.float64, "fp32"),
+                                           (np.float32, "native"), (np.float32, "bf16")])
+def test_bsr_block_rows_around_the_whole_warp_length(bs, layout, dtype, storage):
+    """Block rows just below, at and above 16 steps of 1, 2 and 4 lane sets, in
+    every position of a warp, beside empty ones, a last one alone in its warp;
+    from arrays and converted from CSR; x off a 16-byte boundary."""
+    import torch
+
+    rng = np.random.default_rng(bs)
+    nb = 700
+    lens = [0, 16, 17, 31, 32, 33, 0, 63, 64, 65, 1, 127, 128, 129, 500, 2] + [3] * 41
+    lens += list(rng.integers(0, 5, 60)) + [600, 0, 257]
+    rp, c, _ = csr_of_lengths(lens, nb, rng)
+    v = (rng.integers(-128, 129, int(rp[-1]) * bs * bs) / 64).astype(dtype)  # BF16 holds them
+    v[v == 0] = 1
+    m, n = len(lens) * bs, nb * bs
+    A = pls.SpMat.bsr(layout, m, n, bs, rp, c, v)
+    A.set_storage({"native": pls.STORAGE_NATIVE, "fp32": pls.STORAGE_FP32, "bf16": pls.STORAGE_BF16}[storage])
+    mats = [A]
+    if storage == "native":
+        _, _, srp, sc, sv = pls.SpMat.bsr(layout, m, n, bs, rp, c, v).export_csr()
+        mats.append(pls.SpMat.csr(m, n, srp, sc, sv).to_bsr(bs, layout))
+    x, y0 = W.uniform_vector(n + 1, 4).astype(dtype), W.uniform_vector(m, 5).astype(dtype)
+    xd = torch.tensor(x, device="cuda")
+    # FP32: block rows of at most 600 blocks, 4800 terms, in chains of at most a
+    # tenth of them on one lane: 480 * 2^-24
+    tol = 1e-12 if dtype == np.float64 and storage == "native" else 3e-5
+    v64 = v.astype(np.float64)
+    for off in (0, 1):
+        xs = x[off:off + n].astype(np.float64)
+        ref = oracle.bsr_spmv(rp, c, v64, bs, layout, xs, y=y0.astype(np.float64), alpha=0.5, beta=2.0)
+        scale = 0.5 * oracle.bsr_spmv(rp, c, np.abs(v64), bs, layout, np.abs(xs)) + 2 * np.abs(y0.astype(np.float64))
+        for M in mats:
+            yd = torch.tensor(y0, device="cuda")
+            torch.cuda.synchronize()
+            M.spmv_dev(xd.data_ptr() + off * x.itemsize, yd.data_ptr(), 0.5, 2.0)
+            torch.cuda.synchronize()
+            check(yd.cpu().numpy(), ref, scale, tol)

@@ -494,10 +494,10 @@ def test_chained_products_read_what_the_product_before_wrote(fmt):
 
 
 def us_per_call(run, n=20):
-    """Device time of one call among n on the current stream."""
+    """Device time of one call among n, on a stream of their own."""
     import torch
 
-    s = torch.cuda.current_stream()
+    s = torch.cuda.Stream()
     for _ in range(3):
         run(s.cuda_stream)
     best = np.inf
@@ -512,7 +512,7 @@ def us_per_call(run, n=20):
     return best
 
 
-def bsr_product(A, m, n, dtype):
+def product(A, m, n, dtype):
     import torch
 
     x = torch.zeros(n, dtype=dtype, device="cuda")
@@ -538,7 +538,7 @@ def test_bsr_long_block_row_beside_short_ones(bs):
         rp[1:] = np.cumsum(lens)
         c = rng.integers(0, nb, int(rp[-1])).astype(np.int32)
         A = pls.SpMat.bsr(pls.ROW_MAJOR, mb * bs, nb * bs, bs, rp, c, rng.uniform(-1, 1, len(c) * bs * bs))
-        times.append(us_per_call(bsr_product(A, mb * bs, nb * bs, torch.float64)))
+        times.append(us_per_call(product(A, mb * bs, nb * bs, torch.float64)))
     assert times[1] <= 2 * times[0] + 20
 
 

@@ -109,8 +109,8 @@ __device__ __forceinline__ float ld_keep(const float *p, uint64_t pol) {
 // kernel may start while the kernel before it on the stream drains, instead of
 // after it, so the launch ramp, the row pointers' first loads and the tail of
 // short products overlap. chain_next says that the next kernel may start once
-// every thread of this grid has called it or left: first thing in a kernel of
-// many even CTAs, late where CTAs differ (k_sell). chain_wait returns when the
+// every thread of this grid has called it or left: after a thread's sum (k_sell,
+// k_csr_vector), or first thing where that measured no worse (k_bsr_vec). chain_wait returns when the
 // grid before is complete and its memory visible; what a kernel reads before
 // it is written by no kernel that calls chain_next (matrix data: creation,
 // updates and tuning use ordinary launches). The vector x may be the result of the product before, and y the

@@ -68,24 +68,32 @@ SpmvConfig default_config(const Mat *A) {
 // Each lane has a group of 4 entries in flight: as many lanes as cover the
 // longest row in one round trip, but no more than two for every three entries
 // of the mean row, since lanes past a row's end are idle slots, and at most 16
-// (a warp per row from a mean of 256). Where rows are long enough for the
-// whole-warp part (kCsrLongGroups), the lanes are for the short rows that most
-// rows of such a matrix are, and a quarter of the mean is the better size.
-// Measured (us; the power of two below the mean -> this rule): 5-point
-// Laplacian 2000^2 123 (4) -> 69 (2; 1 lane: 76), 27-point stencil 110^3
-// 145 (16) -> 85 (8; 4: 88), random 500,009 x 17 64 (16) -> 47 (8; 4: 53),
-// 100,009 x 32 27 (32) -> 21 (16; 8: 22), 311,479 FP32 rows of 12 on average
-// and up to 30 entries 22.8 (8) -> 22.8 (4: 23.8), bands of 129 118 (32) -> 87
-// (16); power-law rows of mean 16: 1 M 182 (16) -> 120 (4; 8: 137), 30,000
-// 50 (16) -> 34.
+// (a warp per row from a mean of 192: 201 entries in every one of 250,000 rows
+// take 16 lanes 4 round trips and 230 us, 32 lanes 2 and 201 us; bands of 161
+// 78 and 89 us). Where rows are long enough for the whole-warp part
+// (kCsrLongGroups), the lanes are for the short rows that most rows of such a
+// matrix are: a half to a third of the mean, and no whole-warp part from a mean
+// of 80 (32 lanes). Measured (us; the power of two below the mean -> this
+// rule): 5-point Laplacian 2000^2 123 (4) -> 69 (2; 1 lane: 76), 27-point
+// stencil 110^3 145 (16) -> 85 (8; 4: 88), random 500,009 x 17 64 (16) -> 47
+// (8; 4: 53), 100,009 x 32 27 (32) -> 21 (16; 8: 22), 311,479 FP32 rows of 12
+// on average and up to 30 entries 22.8 (8) -> 22.8 (4: 23.8), bands of 129 118
+// (32) -> 87 (16). Long rows, 300,000 of geometric length, mean 6: 17.0 (4) ->
+// 16.4 (2; 1: 20.2, 4: 15.4), 14: 30.9 (8) -> 28.8 (4; 2: 33.7, 8: 29.6), 24:
+// 49.9 (16) -> 46.6 (8; 4: 46.7), 64: 103.9 (32) -> 100.2 (16; 8: 98.7, FP32
+// 16 85.8, 8 88.8), 100: 138.8 (32) -> 137.0 (32; 16: 143.7); power-law rows
+// of mean 16: 1 M 190 (16) -> 119 (4; 2: 118, 8: 133), 30,000 45 (16) -> 16
+// (4; 2: 19.8).
 int csr_lanes(const CsrDev &c, int32_t rows) {
   const double mean = rows > 0 ? (double)c.nnz / rows : 1.0;
-  if (mean >= 256)
+  if (mean >= 192)
     return 32;
   int t = 1;
   while (t < 16 && 4 * t < c.max_row && 2 * t <= mean / 1.5)
     t *= 2;
-  return c.max_row > csr_long_len(t) ? std::min(16, pow2_floor(mean / 4)) : t;
+  if (c.max_row > csr_long_len(t))
+    t = mean >= 80 ? 32 : mean >= 48 ? 16 : mean >= 20 ? 8 : mean >= 9 ? 4 : mean >= 5 ? 2 : 1;
+  return t;
 }
 
 // Make cfg the active SpMV configuration: build the SELL layout or the

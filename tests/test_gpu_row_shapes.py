@@ -582,3 +582,25 @@ def test_bsr_block_rows_around_the_whole_warp_length(bs, layout, dtype, storage)
             M.spmv_dev(xd.data_ptr() + off * x.itemsize, yd.data_ptr(), 0.5, 2.0)
             torch.cuda.synchronize()
             check(yd.cpu().numpy(), ref, scale, tol)
+
+
+@pytest.mark.parametrize("lengths,mean,rows", [("geometric", 6, 300_000), ("geometric", 14, 300_000),
+                                               ("geometric", 40, 100_000), ("even", 201, 60_000)])
+def test_csr_default_lanes_near_the_best_forced_ones(lengths, mean, rows):
+    """The lanes chosen for a handle that was not optimized, against every lane
+    count forced: within 15% of the fastest (timing spread a few percent)."""
+    import torch
+
+    rng = np.random.default_rng(mean)
+    lens = np.full(rows, mean) if lengths == "even" else rng.geometric(1 / (mean + 1), rows) - 1
+    rp = np.zeros(rows + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    c = rng.integers(0, rows, int(rp[-1])).astype(np.int32)
+    A = pls.SpMat.csr(rows, rows, rp, c, rng.uniform(-1, 1, len(c)))
+    run = product(A, rows, rows, torch.float64)
+    default = us_per_call(run)
+    forced = {}
+    for lanes in (1, 2, 4, 8, 16, 32):
+        assert A.force_config(pls.KIND_CSR, 0, 0, lanes) == 0 and A.optimize() == 0
+        forced[lanes] = us_per_call(run)
+    assert default <= 1.15 * min(forced.values()), (default, forced)

@@ -239,7 +239,7 @@ perflibs_status_t create_csr(Mat **out, int32_t m, int32_t n, const int32_t *row
     // Indices are checked before any kernel uses them (the reference reads
     // them as they are).
     const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(),
-                                      s, &c.max_row);
+                                      s, &c.max_row, &c.reach);
     if (bad.first >= 0)
       return param_error(A, 4, "row_ptr decreases or leaves [0, nnz] at row " + std::to_string(bad.first));
     if (bad.second >= 0)
@@ -544,7 +544,7 @@ constexpr int kMaxBands = 8;
 constexpr int kMaxHostBands = 64;  // bound of an explicit band count
 
 template <class X>
-int band_count(Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen, cudaStream_t s) {
+int band_count(const Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen) {
   if (trans != PERFLIBS_SPARSE_OPERATION_NOTRANS || alpha == X(0) || xlen == 0)
     return 1;
   if (A->fmt != Fmt::SELL && A->fmt != Fmt::CSR)
@@ -554,8 +554,7 @@ int band_count(Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen, cudaStrea
   const int64_t bytes = ylen * (int64_t)sizeof(X);
   if (bytes < 2 * kLocalBandBytes)
     return 1;
-  csr_find_reach(A->csr, A->m, A->ybuf.as<int32_t>(), s);  // ybuf is not in use yet
-  const bool local = 2 * csr_reach(A->csr, A->m, A->m / kMaxBands) <= xlen;
+  const bool local = 2 * csr_reach(A->csr, A->m, A->n, A->m / kMaxBands) <= xlen;
   return (int)std::max<int64_t>(
       1, std::min<int64_t>(kMaxBands, bytes / (local ? kLocalBandBytes : kBandBytes)));
 }
@@ -581,7 +580,6 @@ bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X 
   const size_t nb = bands->size();
   if (nb < 2)
     return false;
-  csr_find_reach(A->csr, A->m, A->ybuf.as<int32_t>(), s);
   BandLanes &L = A->lanes;
   X *xd = A->xbuf.as<X>();
   X *yd = A->ybuf.as<X>();
@@ -610,14 +608,15 @@ bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X 
           cudaStreamSynchronize(q);
     }
   } drain{{u, s, c}};
-  // Events [0, nb): a band's kernels done; nb: work queued on the handle's
-  // stream before this call; nb + 1 + i: band i's upload done.
-  PLS_CUDA(cudaEventRecord(L.event(nb), s));
-  PLS_CUDA(cudaStreamWaitEvent(u, L.event(nb), 0));
+  // A wait takes the event as it was last recorded, so band i's event serves in
+  // turn for its upload and for its kernels, and band 0's before both for the
+  // work queued on the handle's stream before this call.
+  PLS_CUDA(cudaEventRecord(L.event(0), s));
+  PLS_CUDA(cudaStreamWaitEvent(u, L.event(0), 0));
   int64_t have = 0;  // elements of x uploaded
   for (size_t i = 0; i < nb; ++i) {
     const RowBand &b = (*bands)[i];
-    const int64_t need = shared ? xlen : csr_reach(A->csr, A->m, b.r1);
+    const int64_t need = shared ? xlen : csr_reach(A->csr, A->m, A->n, b.r1);
     if (need > have)
       PLS_CUDA(cudaMemcpyAsync(xd + have, x_host + have, sizeof(X) * (size_t)(need - have),
                                cudaMemcpyHostToDevice, u));
@@ -627,8 +626,8 @@ bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X 
       PLS_CUDA(cudaMemcpyAsync(yd + b.r0, y_host + b.r0, sizeof(X) * (size_t)(b.r1 - b.r0),
                                cudaMemcpyHostToDevice, u));
     if (need > have || beta != X(0)) {
-      PLS_CUDA(cudaEventRecord(L.event(nb + 1 + i), u));
-      PLS_CUDA(cudaStreamWaitEvent(s, L.event(nb + 1 + i), 0));
+      PLS_CUDA(cudaEventRecord(L.event(i), u));
+      PLS_CUDA(cudaStreamWaitEvent(s, L.event(i), 0));
     }
     have = std::max(have, need);
     if (A->fmt == Fmt::SELL)
@@ -669,8 +668,8 @@ perflibs_status_t spmv_exec_host(int trans, X alpha, Mat *A, const X *x, X beta,
     if (ylen == 0)
       return PERFLIBS_STATUS_SUCCESS;
     A->xbuf.reserve(sizeof(X) * std::max<int64_t>(xlen, 1));
-    A->ybuf.reserve(std::max<size_t>(sizeof(X) * ylen, sizeof(int32_t) * kReachParts));
-    const int n_bands = band_count<X>(A, trans, alpha, xlen, ylen, s);
+    A->ybuf.reserve(sizeof(X) * ylen);
+    const int n_bands = band_count<X>(A, trans, alpha, xlen, ylen);
     if (n_bands > 1 && spmv_banded<X>(A, n_bands, alpha, x, xlen, beta, y, s))
       return PERFLIBS_STATUS_SUCCESS;
     if (xlen > 0)
@@ -1726,6 +1725,12 @@ perflibs_status_t perflibs_spmv_optimize(perflibs_spmat_t A) {
     tune_spmv(A);
     A->tuned = true;
     A->tuned_op = op;
+    // The streams and events of calls with host vectors: some 80 us that the
+    // first such call would take otherwise.
+    const int bands = A->dt == Dt::F64 ? band_count<double>(A, op, 1.0, A->n, A->m)
+                                       : band_count<float>(A, op, 1.0f, A->n, A->m);
+    if (bands > 1)
+      A->lanes.create((size_t)bands);
     return PERFLIBS_STATUS_SUCCESS;
   });
 }
@@ -2292,7 +2297,7 @@ perflibs_status_t perflibs_b200_spmat_create_csr_d_dev(perflibs_spmat_t *out, in
       PLS_LAUNCH_CHECK();
     }
     const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(),
-                                      s, &c.max_row);
+                                      s, &c.max_row, &c.reach);
     if (bad.first >= 0)
       return param_error(A, 4, "row_ptr decreases or leaves [0, nnz] at row " + std::to_string(bad.first));
     if (bad.second >= 0)

@@ -444,7 +444,8 @@ void build_csr_transpose(const CsrDev &c, int32_t m, int32_t n, CsrDev &out,
     PLS_LAUNCH_CHECK();
     PLS_CUDA(cudaStreamSynchronize(s));
   }
-  T.max_row = longest_row(T.row_ptr, T.nnz > 0 ? n : 0, s);
+  check_compressed(n, m, T.nnz, T.row_ptr.as<int32_t>(), T.col.as<int32_t>(), s, &T.max_row,
+                   &T.reach);
   out = std::move(T);
 }
 
@@ -483,27 +484,90 @@ __global__ void k_gather_entries(int64_t nnz, const int32_t *__restrict__ perm,
 
 namespace {
 
-__global__ void k_check_compressed(int32_t rows, int32_t cols, int64_t nnz,
-                                   const int32_t *__restrict__ ptr,
-                                   const int32_t *__restrict__ idx,
-                                   unsigned long long *__restrict__ bad,
-                                   unsigned *__restrict__ longest) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int32_t len = 0;
-  if (i < rows) {
-    const int32_t a = ptr[i], b = ptr[i + 1];
-    if (a < 0 || b < a || b > nnz)
-      atomicMin(bad, (unsigned long long)i);
+// Rows and entries a CTA checks.
+constexpr int kCheckRounds = 8;
+constexpr int kCheckPer = 256 * kCheckRounds;
+
+// What check_compressed finds, all bits set where nothing was found: the first
+// bad row and entry, and (as complements, for atomicMin) the longest row and
+// one past the largest column of each of kReachParts parts of the rows.
+struct Checked {
+  unsigned long long bad_row, bad_entry;
+  unsigned longest, reach[kReachParts];
+};
+
+// The part of the rows whose entries include entry q. Row pointers that
+// decrease give some part or other: their matrix is refused.
+__device__ __forceinline__ int part_of_entry(const int32_t *__restrict__ ptr, int32_t rows,
+                                             int32_t per, int64_t q) {
+  int lo = 0, hi = kReachParts;  // the last part that starts at or before q
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if ((int64_t)mid * per < rows && ptr[mid * per] <= q)
+      lo = mid;
     else
-      len = b - a;
+      hi = mid;
+  }
+  return lo;
+}
+
+template <bool REACH>
+__global__ void __launch_bounds__(256)
+    k_check_compressed(int32_t rows, int32_t cols, int64_t nnz, const int32_t *__restrict__ ptr,
+                       const int32_t *__restrict__ idx, int32_t per, Checked *__restrict__ out) {
+  __shared__ int ends[2];
+  __shared__ unsigned tops[8];
+  const int64_t i0 = (int64_t)blockIdx.x * kCheckPer;
+  if (REACH && threadIdx.x < 2 && i0 < nnz)
+    ends[threadIdx.x] = part_of_entry(ptr, rows, per,
+                                      threadIdx.x ? min(i0 + kCheckPer, nnz) - 1 : i0);
+  int32_t len = 0;
+#pragma unroll
+  for (int u = 0; u < kCheckRounds; ++u) {
+    const int64_t i = i0 + u * 256 + threadIdx.x;
+    if (i < rows) {
+      const int32_t a = ptr[i], b = ptr[i + 1];
+      if (a < 0 || b < a || b > nnz)
+        atomicMin(&out->bad_row, (unsigned long long)i);
+      else
+        len = max(len, b - a);
+    }
   }
   len = __reduce_max_sync(0xffffffffu, len);
   if (len > 0 && (threadIdx.x & 31) == 0)
-    atomicMin(longest, ~(unsigned)len);  // all ones before the first
-  if (i < nnz) {
-    const int32_t c = idx[i];
-    if (c < 0 || c >= cols)
-      atomicMin(bad + 1, (unsigned long long)i);
+    atomicMin(&out->longest, ~(unsigned)len);
+  if (i0 >= nnz)
+    return;
+  __syncthreads();
+  const bool one = REACH && ends[0] == ends[1];  // the CTA's entries lie in one part
+  unsigned top = 0;
+#pragma unroll
+  for (int u = 0; u < kCheckRounds; ++u) {
+    const int64_t i = i0 + u * 256 + threadIdx.x;
+    if (i < nnz) {
+      const int32_t c = idx[i];
+      if (c < 0 || c >= cols) {
+        atomicMin(&out->bad_entry, (unsigned long long)i);
+      } else if (one) {
+        top = max(top, (unsigned)c + 1);
+      } else if (REACH) {
+        unsigned *r = out->reach + part_of_entry(ptr, rows, per, i);
+        if (~((unsigned)c + 1) < *(volatile unsigned *)r)
+          atomicMin(r, ~((unsigned)c + 1));
+      }
+    }
+  }
+  if (!one)
+    return;
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0)
+    tops[threadIdx.x / 32] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w)
+      top = max(top, tops[w]);
+    if (top > 0)
+      atomicMin(out->reach + ends[0], ~top);
   }
 }
 
@@ -512,27 +576,37 @@ __global__ void k_check_compressed(int32_t rows, int32_t cols, int64_t nnz,
 // Structure check of 0-based compressed arrays before any kernel indexes
 // with them: the first row whose pointers are decreasing or outside
 // [0, nnz], and the first entry whose index is outside [0, cols); -1 each
-// when there is none. On the way, the longest row.
+// when there is none. On the way, the longest row and, where asked for, the
+// columns that the rows reach (CsrDev::reach).
 std::pair<int64_t, int64_t> check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                              const int32_t *ptr, const int32_t *idx,
-                                             cudaStream_t s, int32_t *longest) {
+                                             cudaStream_t s, int32_t *longest,
+                                             std::vector<int32_t> *reach) {
   if (longest)
     *longest = 0;
   const int64_t work = std::max<int64_t>(rows, nnz);
   if (work == 0)
     return {-1, -1};
-  DevBuf bad;
-  bad.reserve(24);
-  PLS_CUDA(cudaMemsetAsync(bad.p, 0xff, 24, s));
-  k_check_compressed<<<(unsigned)div_up(work, 256), 256, 0, s>>>(
-      rows, cols, nnz, ptr, idx, bad.as<unsigned long long>(), bad.as<unsigned>() + 4);
+  DevBuf out;
+  out.reserve(sizeof(Checked));
+  PLS_CUDA(cudaMemsetAsync(out.p, 0xff, sizeof(Checked), s));
+  auto kern = reach && rows > 0 ? k_check_compressed<true> : k_check_compressed<false>;
+  kern<<<(unsigned)div_up(work, kCheckPer), 256, 0, s>>>(
+      rows, cols, nnz, ptr, idx, (int32_t)div_up(rows, kReachParts), out.as<Checked>());
   PLS_LAUNCH_CHECK();
-  unsigned long long h[3];
-  PLS_CUDA(cudaMemcpyAsync(h, bad.p, 24, cudaMemcpyDeviceToHost, s));
+  Checked h;
+  PLS_CUDA(cudaMemcpyAsync(&h, out.p, sizeof(h), cudaMemcpyDeviceToHost, s));
   PLS_CUDA(cudaStreamSynchronize(s));
   if (longest)
-    *longest = (int32_t) ~(unsigned)h[2];
-  return {h[0] == ~0ull ? -1 : (int64_t)h[0], h[1] == ~0ull ? -1 : (int64_t)h[1]};
+    *longest = (int32_t)~h.longest;
+  if (reach) {
+    reach->assign(kReachParts, 0);
+    int32_t top = 0;
+    for (int i = 0; i < kReachParts; ++i)
+      (*reach)[(size_t)i] = top = std::max(top, (int32_t)~h.reach[i]);
+  }
+  return {h.bad_row == ~0ull ? -1 : (int64_t)h.bad_row,
+          h.bad_entry == ~0ull ? -1 : (int64_t)h.bad_entry};
 }
 
 // The entries sorted by (row, column) with a stable radix sort, so equal
@@ -600,7 +674,8 @@ int64_t coo_to_csr(int32_t m, int32_t n, int64_t nnz, const int32_t *row, const 
     PLS_LAUNCH_CHECK();
   }
   PLS_CUDA(cudaStreamSynchronize(s));
-  R.max_row = longest_row(R.row_ptr, R.nnz > 0 ? m : 0, s);
+  check_compressed(m, n, R.nnz, R.row_ptr.as<int32_t>(), R.col.as<int32_t>(), s, &R.max_row,
+                   &R.reach);
   out = std::move(R);
   return -1;
 }
@@ -645,7 +720,8 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
   });
   PLS_LAUNCH_CHECK();
   PLS_CUDA(cudaStreamSynchronize(s));
-  R.max_row = longest_row(R.row_ptr, R.nnz > 0 ? m : 0, s);
+  check_compressed(m, b.nb * b.bs, R.nnz, R.row_ptr.as<int32_t>(), R.col.as<int32_t>(), s,
+                   &R.max_row, &R.reach);
   out = std::move(R);
 }
 

@@ -234,11 +234,11 @@ struct BandPlan {
   }
 };
 
-// The copy streams and events of banded host-buffer calls, created on first
-// use on the handle's GPU: the upload stream brings x (and y) in, piece by
-// piece, and the handle's stream waits for the piece a band needs; event i
-// marks the end of band i's kernels on the handle's stream, and the copy
-// stream waits for it before copying the band's rows of y to the host.
+// The copy streams and events of banded host-buffer calls, created by optimize
+// or on first use on the handle's GPU: the upload stream brings x (and y) in,
+// piece by piece, and the handle's stream waits for the piece a band needs;
+// event i then marks the end of band i's kernels on the handle's stream, and
+// the copy stream waits for it before copying the band's rows of y to the host.
 struct BandLanes {
   cudaStream_t copy = nullptr, upload = nullptr;
   std::vector<cudaEvent_t> ev;
@@ -270,6 +270,11 @@ struct BandLanes {
       ev.push_back(e);
     }
     return ev[i];
+  }
+  void create(size_t bands) {
+    upload_stream();
+    copy_stream();
+    event(bands - 1);
   }
 };
 
@@ -381,6 +386,8 @@ struct DiaDev {
 extern std::atomic<int> g_stage_wait_limit;
 extern std::atomic<int> g_stage_shortfall;
 
+constexpr int kReachParts = 64;
+
 struct CsrDev {
   DevBuf row_ptr, col, vals;  // vals in the API type (authoritative)
   int64_t nnz = 0;
@@ -388,7 +395,7 @@ struct CsrDev {
   int32_t ncols = 0;  // columns (bound of col); 0 when not recorded
   int32_t max_row = INT32_MAX;  // longest row; INT32_MAX when not recorded
   // One past the last column that the rows of each of kReachParts equal parts
-  // read, or any row before them (found on the first banded host-buffer call).
+  // read, or any row before them (found at creation; empty when not recorded).
   std::vector<int32_t> reach;
   Vt vt = Vt::F64;
   // Reduced-precision copy of the values used by the kernels when the
@@ -605,11 +612,8 @@ void csr_plan_bands(CsrDev &c, int32_t m, int n_bands);
 template <class X>
 void spmv_sell_band(const SellDev &s, const RowBand &b, const X *x, X *y, X alpha, X beta,
                     cudaStream_t st);
-// CsrDev::reach (`scratch`: kReachParts device words), and the columns
-// [0, result) that rows [0, r1) read.
-constexpr int kReachParts = 64;
-void csr_find_reach(CsrDev &c, int32_t m, int32_t *scratch, cudaStream_t s);
-int64_t csr_reach(const CsrDev &c, int32_t m, int64_t r1);
+// The columns [0, result) that rows [0, r1) of an m x n matrix read.
+int64_t csr_reach(const CsrDev &c, int32_t m, int32_t n, int64_t r1);
 // tpr = 0 runs the long-row split kernels (threshold c.long_threshold).
 template <class X>
 void spmv_csr_band(const CsrDev &c, const RowBand &b, int tpr, const X *x, X *y, X alpha,
@@ -683,10 +687,12 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
                 cudaStream_t s);
 // First bad row (pointers decreasing or outside [0, nnz]) and first bad
 // entry (index outside [0, cols)) of 0-based compressed device arrays, -1
-// when none; the longest row (0 without rows) in *longest.
+// when none; the longest row (0 without rows) in *longest, and CsrDev::reach
+// in *reach.
 std::pair<int64_t, int64_t> check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                              const int32_t *ptr, const int32_t *idx,
-                                             cudaStream_t s, int32_t *longest = nullptr);
+                                             cudaStream_t s, int32_t *longest = nullptr,
+                                             std::vector<int32_t> *reach = nullptr);
 // COO (0-based device arrays, any order, duplicates allowed) -> CSR sorted by
 // (row, column), duplicates kept in input order. Returns -1, or the first
 // entry whose row or column is out of range (then `out` is untouched).

@@ -655,39 +655,11 @@ void csr_plan_bands(CsrDev &c, int32_t m, int n_bands) {
   PLS_CUDA(cudaDeviceSynchronize());
 }
 
-// Warp per row: the row's largest column + 1 into its part's maximum.
-__global__ void k_reach(int32_t m, int32_t per, const int32_t *__restrict__ rp,
-                        const int32_t *__restrict__ col, int32_t *__restrict__ reach) {
-  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  if (row >= m)
-    return;
-  int32_t hi = 0;
-  for (int32_t j = rp[row] + (int32_t)(threadIdx.x & 31); j < rp[row + 1]; j += 32)
-    hi = max(hi, col[j] + 1);
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  if ((threadIdx.x & 31) == 0 && hi > reach[row / per])
-    atomicMax(reach + row / per, hi);
-}
-
-void csr_find_reach(CsrDev &c, int32_t m, int32_t *scratch, cudaStream_t s) {
-  if (!c.reach.empty() || m <= 0)
-    return;
-  std::vector<int32_t> h(kReachParts, 0);
-  PLS_CUDA(cudaMemsetAsync(scratch, 0, sizeof(int32_t) * kReachParts, s));
-  k_reach<<<(unsigned)div_up((int64_t)m * 32, 256), 256, 0, s>>>(
-      m, (int32_t)div_up(m, kReachParts), c.row_ptr.as<int32_t>(), c.col.as<int32_t>(), scratch);
-  PLS_LAUNCH_CHECK();
-  PLS_CUDA(cudaMemcpyAsync(h.data(), scratch, sizeof(int32_t) * kReachParts,
-                           cudaMemcpyDeviceToHost, s));
-  PLS_CUDA(cudaStreamSynchronize(s));
-  for (int i = 1; i < kReachParts; ++i)
-    h[(size_t)i] = std::max(h[(size_t)i], h[(size_t)i - 1]);
-  c.reach = std::move(h);
-}
-
-int64_t csr_reach(const CsrDev &c, int32_t m, int64_t r1) {
-  if (r1 <= 0)
+int64_t csr_reach(const CsrDev &c, int32_t m, int32_t n, int64_t r1) {
+  if (r1 <= 0 || c.nnz == 0)
     return 0;
+  if (c.reach.empty())
+    return n;
   const int64_t part = (std::min<int64_t>(r1, m) - 1) / div_up(m, kReachParts);
   return c.reach[(size_t)std::min<int64_t>(part, kReachParts - 1)];
 }

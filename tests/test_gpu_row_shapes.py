@@ -604,3 +604,61 @@ def test_csr_default_lanes_near_the_best_forced_ones(lengths, mean, rows):
         assert A.force_config(pls.KIND_CSR, 0, 0, lanes) == 0 and A.optimize() == 0
         forced[lanes] = us_per_call(run)
     assert default <= 1.15 * min(forced.values()), (default, forced)
+
+
+def kernels_of(call):
+    """The kernels that a call launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return sorted(e.name for e in p.events() if "pls::" in e.name)
+
+
+@pytest.mark.parametrize("create", ["csr", "coo", "csc", "bsr_trans"])
+def test_first_host_call_launches_what_later_ones_do(create):
+    """What the calls need to know of the matrix is found at its creation: the
+    first call with host vectors runs the products alone."""
+    import torch
+
+    m, n, rp, c, v = W.laplacian_2d(800)  # symmetric: its CSC arrays are its CSR arrays
+    rows = np.repeat(np.arange(m, dtype=np.int32), np.diff(rp))
+    A = {"csr": lambda: pls.SpMat.csr(m, n, rp, c, v), "coo": lambda: pls.SpMat.coo(m, n, rows, c, v),
+         "csc": lambda: pls.SpMat.csc(m, n, c, rp, v),
+         "bsr_trans": lambda: pls.SpMat.csr(m, n, rp, c, v).to_bsr(2)}[create]()
+    x = torch.tensor(W.uniform_vector(n, 3)).pin_memory().numpy()
+    y = torch.zeros(m, dtype=torch.float64).pin_memory().numpy()
+    if create == "bsr_trans":  # becomes a CSR handle
+        A.spmv(x, y, trans=pls.OPERATION_TRANS)
+    kernels_of(lambda: None)
+    first, second = [kernels_of(lambda: A.spmv(x, y)) for _ in range(2)]
+    assert len(second) > 1 and first == second
+    check(y, oracle.csr_spmv(rp, c, v, x), oracle.csr_absdot(rp, c, v, x), 1e-12)
+
+
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 3000, 40_000])
+def test_columns_reached_by_the_first_rows(rows):
+    """x goes to the GPU up to the columns that the rows so far read: matrices
+    whose rows need the most (one column far ahead of the rest at every sixth
+    row, all zero rows between), in as many bands as there are, against whole
+    products; entries of one part, of several and of all parts of the rows in
+    one CTA of the check."""
+    rng = np.random.default_rng(rows)
+    n = rows + 700
+    lens = np.where(np.arange(rows) % 6 == 5, 9, np.where(np.arange(rows) % 6 < 3, 0, 2))
+    rp = np.zeros(rows + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    r = np.repeat(np.arange(rows), lens)
+    c = np.minimum(r + rng.integers(0, 600, len(r)), n - 1)
+    v = rng.standard_normal(len(c))
+    x = W.uniform_vector(n, 2)
+    order = np.lexsort((c, r))
+    c = c[order].astype(np.int32)
+    for base in (0, 1):
+        A = pls.SpMat.csr(rows, n, rp + base, c + base, v)
+        A.set_host_bands(min(64, rows))
+        A.spmv(np.full(n, np.nan))  # what is not copied is NaN
+        check(A.spmv(x), oracle.csr_spmv(rp, c, v, x), oracle.csr_absdot(rp, c, v, x), 1e-12)

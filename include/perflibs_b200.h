@@ -161,10 +161,11 @@ perflibs_status_t perflibs_b200_spmat_set_spmm_path(perflibs_spmat_t A, int32_t 
  * the first band hide under the device-to-host copy. Applies to NOTRANS
  * with CSR or SELL-C-sigma kernels; every row is summed exactly as in one
  * launch. n_bands = 0 (default) splits results of 8 MB and more into bands
- * of at least 4 MB, up to 8, and where the first eighth of the rows reads at
- * most half of x, results of 2 MB and more into bands of at least 1 MB, up to
- * 8; x is then copied in as the bands need it. 1 turns banding off; 2..64 asks for that many
- * (SELL bands are whole sort windows, so there may be fewer). */
+ * of at least 4 MB, up to 8. Where x and y are pinned and the first eighth of
+ * the rows reads at most half of x, it splits results of 2 MB and more into
+ * bands of at least 1 MB, up to 8. Pinned x is copied in as the bands need
+ * it. 1 turns banding off; 2..64 asks for that many (SELL bands are whole
+ * sort windows, so there may be fewer). */
 perflibs_status_t perflibs_b200_spmat_set_host_bands(perflibs_spmat_t A, int32_t n_bands);
 
 /* Bands the handle's last host-buffer SpMV ran in; 0 when it ran as one

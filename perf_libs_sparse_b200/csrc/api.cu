@@ -537,14 +537,24 @@ template <class X> bool matches(const Mat *A) {
 // copy runs beside y's in the other direction; smaller bands then start y's
 // copy earlier. A 5-point Laplacian of 1000^2 (8 MB each way, pinned), 2 bands
 // behind x's copy -> 7 bands with x in pieces: 331 -> 302 us; on a host whose
-// uploads ran at 19 GB/s 551 -> 320 us.
+// uploads ran at 19 GB/s 551 -> 320 us. Only where both vectors are pinned:
+// copies of pageable memory go through the host one after another, and more of
+// them take longer (1000^2 pageable 1006 us in one piece, 1264 us in 7).
 constexpr int64_t kBandBytes = 4 << 20;
 constexpr int64_t kLocalBandBytes = 1 << 20;
 constexpr int kMaxBands = 8;
 constexpr int kMaxHostBands = 64;  // bound of an explicit band count
 
+bool host_pinned(const void *p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) == cudaSuccess)
+    return at.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+
 template <class X>
-int band_count(const Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen) {
+int band_count(const Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen, bool pinned) {
   if (trans != PERFLIBS_SPARSE_OPERATION_NOTRANS || alpha == X(0) || xlen == 0)
     return 1;
   if (A->fmt != Fmt::SELL && A->fmt != Fmt::CSR)
@@ -554,7 +564,8 @@ int band_count(const Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen) {
   const int64_t bytes = ylen * (int64_t)sizeof(X);
   if (bytes < 2 * kLocalBandBytes)
     return 1;
-  const bool local = 2 * csr_reach(A->csr, A->m, A->n, A->m / kMaxBands) <= xlen;
+  const bool local =
+      pinned && 2 * csr_reach(A->csr, A->m, A->n, A->m / kMaxBands) <= xlen;
   return (int)std::max<int64_t>(
       1, std::min<int64_t>(kMaxBands, bytes / (local ? kLocalBandBytes : kBandBytes)));
 }
@@ -562,13 +573,13 @@ int band_count(const Mat *A, int trans, X alpha, int64_t xlen, int64_t ylen) {
 // The bands' kernels run in band order on the handle's stream, each after the
 // piece of x (with beta != 0 also its rows of y) that the upload stream brings
 // it; a band's event releases the copy of its rows on the copy stream. With
-// pageable host memory a copy may block the host, so then all kernels are
-// queued before the first copy back. (Bands on several streams at once
-// measured slower: the first band then shares the GPU with the others and its
-// copy starts later.)
+// pageable host memory a copy may block the host, so then x and y come in
+// whole and all kernels are queued before the first copy back. (Bands on
+// several streams at once measured slower: the first band then shares the GPU
+// with the others and its copy starts later.)
 template <class X>
 bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X beta, X *y_host,
-                 cudaStream_t s) {
+                 bool pinned, cudaStream_t s) {
   const std::vector<RowBand> *bands;
   if (A->fmt == Fmt::SELL) {
     sell_plan_bands(A->sell, A->m, n_bands);
@@ -589,10 +600,7 @@ bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X 
   // y's rows may go back while x is still read: all of x first when they share
   // memory.
   const bool shared = x_host < y_host + A->m && y_host < x_host + xlen;
-  cudaPointerAttributes at{};
-  const bool pinned = cudaPointerGetAttributes(&at, y_host) == cudaSuccess &&
-                      at.type == cudaMemoryTypeHost;
-  cudaStream_t c = L.copy_stream(), u = L.upload_stream();
+  cudaStream_t c = L.copy_stream(), u = pinned ? L.upload_stream() : s;
   const auto copy_back = [&](size_t i) {
     const RowBand &b = (*bands)[i];
     PLS_CUDA(cudaStreamWaitEvent(c, L.event(i), 0));
@@ -611,21 +619,25 @@ bool spmv_banded(Mat *A, int n_bands, X alpha, const X *x_host, int64_t xlen, X 
   // A wait takes the event as it was last recorded, so band i's event serves in
   // turn for its upload and for its kernels, and band 0's before both for the
   // work queued on the handle's stream before this call.
-  PLS_CUDA(cudaEventRecord(L.event(0), s));
-  PLS_CUDA(cudaStreamWaitEvent(u, L.event(0), 0));
+  if (pinned) {
+    PLS_CUDA(cudaEventRecord(L.event(0), s));
+    PLS_CUDA(cudaStreamWaitEvent(u, L.event(0), 0));
+  }
   int64_t have = 0;  // elements of x uploaded
   for (size_t i = 0; i < nb; ++i) {
     const RowBand &b = (*bands)[i];
-    const int64_t need = shared ? xlen : csr_reach(A->csr, A->m, A->n, b.r1);
+    const int64_t need =
+        shared || !pinned ? xlen : csr_reach(A->csr, A->m, A->n, b.r1);
     if (need > have)
       PLS_CUDA(cudaMemcpyAsync(xd + have, x_host + have, sizeof(X) * (size_t)(need - have),
                                cudaMemcpyHostToDevice, u));
     // With beta = 0 every kernel writes all of y without reading it (the
     // reference's y = alpha*A*x: old values, NaN included, do not propagate).
-    if (beta != X(0))
-      PLS_CUDA(cudaMemcpyAsync(yd + b.r0, y_host + b.r0, sizeof(X) * (size_t)(b.r1 - b.r0),
+    const int64_t y1 = pinned ? b.r1 : i == 0 ? A->m : b.r0;
+    if (beta != X(0) && y1 > b.r0)
+      PLS_CUDA(cudaMemcpyAsync(yd + b.r0, y_host + b.r0, sizeof(X) * (size_t)(y1 - b.r0),
                                cudaMemcpyHostToDevice, u));
-    if (need > have || beta != X(0)) {
+    if (pinned && (need > have || beta != X(0))) {
       PLS_CUDA(cudaEventRecord(L.event(i), u));
       PLS_CUDA(cudaStreamWaitEvent(s, L.event(i), 0));
     }
@@ -669,8 +681,11 @@ perflibs_status_t spmv_exec_host(int trans, X alpha, Mat *A, const X *x, X beta,
       return PERFLIBS_STATUS_SUCCESS;
     A->xbuf.reserve(sizeof(X) * std::max<int64_t>(xlen, 1));
     A->ybuf.reserve(sizeof(X) * ylen);
-    const int n_bands = band_count<X>(A, trans, alpha, xlen, ylen);
-    if (n_bands > 1 && spmv_banded<X>(A, n_bands, alpha, x, xlen, beta, y, s))
+    const bool may_band =
+        A->host_bands > 1 || ylen * (int64_t)sizeof(X) >= 2 * kLocalBandBytes;
+    const bool pinned = may_band && host_pinned(x) && host_pinned(y);
+    const int n_bands = band_count<X>(A, trans, alpha, xlen, ylen, pinned);
+    if (n_bands > 1 && spmv_banded<X>(A, n_bands, alpha, x, xlen, beta, y, pinned, s))
       return PERFLIBS_STATUS_SUCCESS;
     if (xlen > 0)
       PLS_CUDA(cudaMemcpyAsync(A->xbuf.p, x, sizeof(X) * xlen, cudaMemcpyHostToDevice, s));
@@ -1727,8 +1742,8 @@ perflibs_status_t perflibs_spmv_optimize(perflibs_spmat_t A) {
     A->tuned_op = op;
     // The streams and events of calls with host vectors: some 80 us that the
     // first such call would take otherwise.
-    const int bands = A->dt == Dt::F64 ? band_count<double>(A, op, 1.0, A->n, A->m)
-                                       : band_count<float>(A, op, 1.0f, A->n, A->m);
+    const int bands = A->dt == Dt::F64 ? band_count<double>(A, op, 1.0, A->n, A->m, true)
+                                       : band_count<float>(A, op, 1.0f, A->n, A->m, true);
     if (bands > 1)
       A->lanes.create((size_t)bands);
     return PERFLIBS_STATUS_SUCCESS;

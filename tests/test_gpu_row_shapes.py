@@ -662,3 +662,24 @@ def test_columns_reached_by_the_first_rows(rows):
         A.set_host_bands(min(64, rows))
         A.spmv(np.full(n, np.nan))  # what is not copied is NaN
         check(A.spmv(x), oracle.csr_spmv(rp, c, v, x), oracle.csr_absdot(rp, c, v, x), 1e-12)
+
+
+@pytest.mark.parametrize("grid", [600, 1000, 1100])
+def test_pageable_vectors_are_banded_by_size_alone(grid):
+    """x in pieces and bands of 1 MB are for pinned vectors: with one of the two
+    pageable, bands of 4 MB behind all of x."""
+    import torch
+
+    m, n, rp, c, v = W.laplacian_2d(grid)
+    A = pls.SpMat.csr(m, n, rp, c, v)
+    xp, yp = W.uniform_vector(n, 3), W.uniform_vector(m, 4)
+    xq, yq = torch.tensor(xp).pin_memory().numpy(), torch.tensor(yp).pin_memory().numpy()
+    ref = oracle.csr_spmv(rp, c, v, xp, y=yp, alpha=2.0, beta=-0.5)
+    scale = 2 * oracle.csr_absdot(rp, c, v, xp) + 0.5 * np.abs(yp)
+    used = []
+    for x, y in ((xq, yq), (xp, yp), (xp, yq), (xq, yp)):
+        y = y.copy() if y is yp else torch.tensor(yp).pin_memory().numpy()
+        check(A.spmv(x, y, alpha=2.0, beta=-0.5), ref, scale, 1e-12)
+        used.append(A.host_bands_used())
+    assert used[0] == m * 8 // 2 ** 20 if m * 8 < 2 ** 23 else used[0] == 8
+    assert used[1:] == [m * 8 // 2 ** 22 if m * 8 >= 2 ** 23 else 0] * 3

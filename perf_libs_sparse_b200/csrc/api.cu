@@ -234,16 +234,18 @@ perflibs_status_t create_csr(Mat **out, int32_t m, int32_t n, const int32_t *row
     c.ncols = n;
     c.vt = native_vt(A->dt);
     upload_index(c.row_ptr, row_ptr, (int64_t)m + 1, A->index_base, s);
+    csr_reserve_columns(c, m);
     upload_index(c.col, col, A->nnz, A->index_base, s);
     upload(c.vals, vals, sizeof(T) * A->nnz, s);
     // Indices are checked before any kernel uses them (the reference reads
     // them as they are).
     const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(),
-                                      s, &c.max_row, &c.reach);
+                                      s, nullptr, &c);
     if (bad.first >= 0)
       return param_error(A, 4, "row_ptr decreases or leaves [0, nnz] at row " + std::to_string(bad.first));
     if (bad.second >= 0)
       return param_error(A, 5, "col_indx[" + std::to_string(bad.second) + "] is outside [0, n)");
+    csr_list_wide_rows(c, m, s);
     A->cfg = default_config(A);
     return PERFLIBS_STATUS_SUCCESS;
   });
@@ -2297,7 +2299,7 @@ perflibs_status_t perflibs_b200_spmat_create_csr_d_dev(perflibs_spmat_t *out, in
     c.ncols = n;
     c.vt = Vt::F64;
     c.row_ptr.reserve(4 * ((size_t)m + 1));
-    c.col.reserve(std::max<size_t>(4 * A->nnz, 16));
+    csr_reserve_columns(c, m);
     c.vals.reserve(std::max<size_t>(8 * A->nnz, 16));
     PLS_CUDA(cudaMemcpyAsync(c.row_ptr.p, row_ptr, 4 * ((size_t)m + 1), cudaMemcpyDeviceToDevice, s));
     if (A->nnz) {
@@ -2312,11 +2314,12 @@ perflibs_status_t perflibs_b200_spmat_create_csr_d_dev(perflibs_spmat_t *out, in
       PLS_LAUNCH_CHECK();
     }
     const auto bad = check_compressed(m, n, A->nnz, c.row_ptr.as<int32_t>(), c.col.as<int32_t>(),
-                                      s, &c.max_row, &c.reach);
+                                      s, nullptr, &c);
     if (bad.first >= 0)
       return param_error(A, 4, "row_ptr decreases or leaves [0, nnz] at row " + std::to_string(bad.first));
     if (bad.second >= 0)
       return param_error(A, 5, "col_indx[" + std::to_string(bad.second) + "] is outside [0, n)");
+    csr_list_wide_rows(c, m, s);
     A->cfg = default_config(A);
     return PERFLIBS_STATUS_SUCCESS;
   });

@@ -444,8 +444,8 @@ void build_csr_transpose(const CsrDev &c, int32_t m, int32_t n, CsrDev &out,
     PLS_LAUNCH_CHECK();
     PLS_CUDA(cudaStreamSynchronize(s));
   }
-  check_compressed(n, m, T.nnz, T.row_ptr.as<int32_t>(), T.col.as<int32_t>(), s, &T.max_row,
-                   &T.reach);
+  check_compressed(n, m, T.nnz, T.row_ptr.as<int32_t>(), T.col.as<int32_t>(), s, nullptr, &T);
+  csr_list_wide_rows(T, n, s);
   out = std::move(T);
 }
 
@@ -489,12 +489,25 @@ constexpr int kCheckRounds = 8;
 constexpr int kCheckPer = 256 * kCheckRounds;
 
 // What check_compressed finds, all bits set where nothing was found: the first
-// bad row and entry, and (as complements, for atomicMin) the longest row and
-// one past the largest column of each of kReachParts parts of the rows.
+// bad row and entry; as complements, for atomicMin, the longest row and one past
+// the largest column of each of kReachParts parts of the rows; and, one less
+// than there are, the rows longer than the threshold in each bucket.
 struct Checked {
   unsigned long long bad_row, bad_entry;
-  unsigned longest, reach[kReachParts];
+  unsigned longest, reach[kReachParts], wide[32];
 };
+
+// Length past which a row is listed: 128 entries, and 8 times the mean.
+int32_t wide_threshold(int32_t rows, int64_t nnz) {
+  constexpr int kWideRow = 128, kWideMean = 8;
+  if (rows <= 0)
+    return INT32_MAX;
+  return (int32_t)std::min<double>(
+      INT32_MAX, std::max<double>(kWideRow, kWideMean * std::ceil((double)nnz / rows)));
+}
+
+// The bucket of a listed row: the last power of two that its length passes.
+__device__ __forceinline__ int wide_bucket(int32_t len) { return 31 - __clz(len - 1); }
 
 // The part of the rows whose entries include entry q. Row pointers that
 // decrease give some part or other: their matrix is refused.
@@ -511,14 +524,15 @@ __device__ __forceinline__ int part_of_entry(const int32_t *__restrict__ ptr, in
   return lo;
 }
 
-template <bool REACH>
+template <bool FACTS>
 __global__ void __launch_bounds__(256)
     k_check_compressed(int32_t rows, int32_t cols, int64_t nnz, const int32_t *__restrict__ ptr,
-                       const int32_t *__restrict__ idx, int32_t per, Checked *__restrict__ out) {
+                       const int32_t *__restrict__ idx, int32_t per, int32_t thr,
+                       Checked *__restrict__ out) {
   __shared__ int ends[2];
   __shared__ unsigned tops[8];
   const int64_t i0 = (int64_t)blockIdx.x * kCheckPer;
-  if (REACH && threadIdx.x < 2 && i0 < nnz)
+  if (FACTS && threadIdx.x < 2 && i0 < nnz)
     ends[threadIdx.x] = part_of_entry(ptr, rows, per,
                                       threadIdx.x ? min(i0 + kCheckPer, nnz) - 1 : i0);
   int32_t len = 0;
@@ -527,10 +541,13 @@ __global__ void __launch_bounds__(256)
     const int64_t i = i0 + u * 256 + threadIdx.x;
     if (i < rows) {
       const int32_t a = ptr[i], b = ptr[i + 1];
-      if (a < 0 || b < a || b > nnz)
+      if (a < 0 || b < a || b > nnz) {
         atomicMin(&out->bad_row, (unsigned long long)i);
-      else
+      } else {
         len = max(len, b - a);
+        if (FACTS && b - a > thr)
+          atomicAdd(out->wide + wide_bucket(b - a), 1u);
+      }
     }
   }
   len = __reduce_max_sync(0xffffffffu, len);
@@ -539,7 +556,7 @@ __global__ void __launch_bounds__(256)
   if (i0 >= nnz)
     return;
   __syncthreads();
-  const bool one = REACH && ends[0] == ends[1];  // the CTA's entries lie in one part
+  const bool one = FACTS && ends[0] == ends[1];  // the CTA's entries lie in one part
   unsigned top = 0;
 #pragma unroll
   for (int u = 0; u < kCheckRounds; ++u) {
@@ -550,7 +567,7 @@ __global__ void __launch_bounds__(256)
         atomicMin(&out->bad_entry, (unsigned long long)i);
       } else if (one) {
         top = max(top, (unsigned)c + 1);
-      } else if (REACH) {
+      } else if (FACTS) {
         unsigned *r = out->reach + part_of_entry(ptr, rows, per, i);
         if (~((unsigned)c + 1) < *(volatile unsigned *)r)
           atomicMin(r, ~((unsigned)c + 1));
@@ -576,37 +593,86 @@ __global__ void __launch_bounds__(256)
 // Structure check of 0-based compressed arrays before any kernel indexes
 // with them: the first row whose pointers are decreasing or outside
 // [0, nnz], and the first entry whose index is outside [0, cols); -1 each
-// when there is none. On the way, the longest row and, where asked for, the
-// columns that the rows reach (CsrDev::reach).
+// when there is none. On the way, the longest row and, where asked for, what
+// a CsrDev records of its rows (max_row, reach, the number of wide rows).
 std::pair<int64_t, int64_t> check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                              const int32_t *ptr, const int32_t *idx,
-                                             cudaStream_t s, int32_t *longest,
-                                             std::vector<int32_t> *reach) {
+                                             cudaStream_t s, int32_t *longest, CsrDev *facts) {
   if (longest)
     *longest = 0;
+  if (facts)
+    facts->max_row = 0;
   const int64_t work = std::max<int64_t>(rows, nnz);
   if (work == 0)
     return {-1, -1};
+  const int32_t thr = wide_threshold(rows, nnz);
   DevBuf out;
   out.reserve(sizeof(Checked));
   PLS_CUDA(cudaMemsetAsync(out.p, 0xff, sizeof(Checked), s));
-  auto kern = reach && rows > 0 ? k_check_compressed<true> : k_check_compressed<false>;
+  auto kern = facts && rows > 0 ? k_check_compressed<true> : k_check_compressed<false>;
   kern<<<(unsigned)div_up(work, kCheckPer), 256, 0, s>>>(
-      rows, cols, nnz, ptr, idx, (int32_t)div_up(rows, kReachParts), out.as<Checked>());
+      rows, cols, nnz, ptr, idx, (int32_t)div_up(rows, kReachParts), thr, out.as<Checked>());
   PLS_LAUNCH_CHECK();
   Checked h;
   PLS_CUDA(cudaMemcpyAsync(&h, out.p, sizeof(h), cudaMemcpyDeviceToHost, s));
   PLS_CUDA(cudaStreamSynchronize(s));
   if (longest)
     *longest = (int32_t)~h.longest;
-  if (reach) {
-    reach->assign(kReachParts, 0);
-    int32_t top = 0;
+  if (facts) {
+    facts->max_row = (int32_t)~h.longest;
+    facts->reach.assign(kReachParts, 0);
+    int32_t top = 0, above = 0;
     for (int i = 0; i < kReachParts; ++i)
-      (*reach)[(size_t)i] = top = std::max(top, (int32_t)~h.reach[i]);
+      facts->reach[(size_t)i] = top = std::max(top, (int32_t)~h.reach[i]);
+    facts->wide_thr = thr;
+    for (int b = 31; b >= 0; --b)
+      facts->wide_above[b] = above += (int32_t)(h.wide[b] + 1u);
   }
   return {h.bad_row == ~0ull ? -1 : (int64_t)h.bad_row,
           h.bad_entry == ~0ull ? -1 : (int64_t)h.bad_entry};
+}
+
+namespace {
+
+// The listed rows, by the power of two that their lengths pass, highest first:
+// next[b] is where bucket b's next row goes.
+__global__ void k_wide_rows(int32_t m, int32_t thr, const int32_t *__restrict__ rp,
+                            int32_t *__restrict__ next, int32_t *__restrict__ rows) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= m)
+    return;
+  const int32_t len = rp[r + 1] - rp[r];
+  if (len > thr)
+    rows[atomicAdd(next + wide_bucket(len), 1)] = (int32_t)r;
+}
+
+}  // namespace
+
+void csr_reserve_columns(CsrDev &c, int32_t m) {
+  c.col.reserve(sizeof(int32_t) * (size_t)(std::max<int64_t>(c.nnz, 1) +
+                                           c.nnz / ((int64_t)wide_threshold(m, c.nnz) + 1) + 32));
+}
+
+void csr_list_wide_rows(CsrDev &c, int32_t m, cudaStream_t s) {
+  if (c.n_wide() == 0)
+    return;
+  // the list, then the buckets' cursors
+  const size_t need = sizeof(int32_t) * ((size_t)c.n_wide() + 32);
+  if (c.col.bytes >= sizeof(int32_t) * (size_t)c.nnz + need) {
+    c.wide_list = c.col.as<int32_t>() + c.nnz;
+  } else {
+    c.wide_rows.reserve(need);
+    c.wide_list = c.wide_rows.as<int32_t>();
+  }
+  int32_t *const next = c.wide_list + c.n_wide();
+  int32_t first[32];
+  for (int b = 0; b < 32; ++b)
+    first[b] = b < 31 ? c.wide_above[b + 1] : 0;
+  PLS_CUDA(cudaMemcpyAsync(next, first, sizeof(first), cudaMemcpyHostToDevice, s));
+  k_wide_rows<<<(unsigned)div_up(m, 256), 256, 0, s>>>(m, c.wide_thr, c.row_ptr.as<int32_t>(),
+                                                       next, c.wide_list);
+  PLS_LAUNCH_CHECK();
+  PLS_CUDA(cudaStreamSynchronize(s));
 }
 
 // The entries sorted by (row, column) with a stable radix sort, so equal
@@ -674,8 +740,8 @@ int64_t coo_to_csr(int32_t m, int32_t n, int64_t nnz, const int32_t *row, const 
     PLS_LAUNCH_CHECK();
   }
   PLS_CUDA(cudaStreamSynchronize(s));
-  check_compressed(m, n, R.nnz, R.row_ptr.as<int32_t>(), R.col.as<int32_t>(), s, &R.max_row,
-                   &R.reach);
+  check_compressed(m, n, R.nnz, R.row_ptr.as<int32_t>(), R.col.as<int32_t>(), s, nullptr, &R);
+  csr_list_wide_rows(R, m, s);
   out = std::move(R);
   return -1;
 }
@@ -721,7 +787,8 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
   PLS_LAUNCH_CHECK();
   PLS_CUDA(cudaStreamSynchronize(s));
   check_compressed(m, b.nb * b.bs, R.nnz, R.row_ptr.as<int32_t>(), R.col.as<int32_t>(), s,
-                   &R.max_row, &R.reach);
+                   nullptr, &R);
+  csr_list_wide_rows(R, m, s);
   out = std::move(R);
 }
 
@@ -860,28 +927,6 @@ int64_t count_blocks(const CsrDev &c, int32_t m, int32_t n, int bs, cudaStream_t
   PLS_CUDA(cudaMemcpyAsync(&last, bid.as<int32_t>() + nnz - 1, 4, cudaMemcpyDeviceToHost, s));
   PLS_CUDA(cudaStreamSynchronize(s));
   return last;
-}
-
-void list_long_rows(const DevBuf &row_ptr, int32_t m, int threshold, DevBuf &rows,
-                    std::vector<int32_t> &lens, cudaStream_t s) {
-  std::vector<int32_t> rp((size_t)m + 1);
-  PLS_CUDA(cudaMemcpyAsync(rp.data(), row_ptr.p, sizeof(int32_t) * rp.size(),
-                           cudaMemcpyDeviceToHost, s));
-  PLS_CUDA(cudaStreamSynchronize(s));
-  std::vector<int32_t> list;
-  for (int32_t r = 0; r < m; ++r)
-    if (rp[r + 1] - rp[r] > threshold)
-      list.push_back(r);
-  std::stable_sort(list.begin(), list.end(), [&](int32_t a, int32_t b) {
-    return rp[a + 1] - rp[a] > rp[b + 1] - rp[b];
-  });
-  lens.clear();
-  for (const int32_t r : list)
-    lens.push_back(rp[r + 1] - rp[r]);
-  rows.reserve(sizeof(int32_t) * std::max<size_t>(list.size(), 1));
-  PLS_CUDA(cudaMemcpyAsync(rows.p, list.data(), sizeof(int32_t) * list.size(),
-                           cudaMemcpyHostToDevice, s));
-  PLS_CUDA(cudaStreamSynchronize(s));
 }
 
 void csr_build_long_rows(CsrDev &c, int32_t m, int threshold, cudaStream_t s) {

@@ -410,11 +410,17 @@ struct CsrDev {
   DevBuf long_rows;
   int n_long = 0;
   int long_threshold = 0;
-  // Rows far longer than the mean, longest first, with their lengths: the
-  // SpMM gives them whole CTAs (found on the first SpMM).
-  bool wide_found = false;
+  // Rows of more than wide_thr entries (128, and 8 times the mean), which the
+  // SpMM gives whole CTAs: listed at creation by the power of two that their
+  // lengths pass, highest first; wide_above[b] of them are longer than 2^b. The
+  // list lies behind the column indices where csr_reserve_columns left room
+  // (0.8% of them at most; an allocation of its own took a creation from device
+  // arrays 0.3 ms), else in wide_rows.
+  int32_t wide_thr = INT32_MAX;
+  int32_t wide_above[32] = {};
+  int32_t *wide_list = nullptr;
   DevBuf wide_rows;
-  std::vector<int32_t> wide_len;
+  int32_t n_wide() const { return wide_above[0]; }
   // Staged-SpMM tiles (built on the first suitable SpMM).
   TileDev tiles;
   DiaDev dia;
@@ -687,12 +693,12 @@ void bsr_to_csr(const BsrDev &b, int32_t m, bool drop_zeros, CsrDev &out,
                 cudaStream_t s);
 // First bad row (pointers decreasing or outside [0, nnz]) and first bad
 // entry (index outside [0, cols)) of 0-based compressed device arrays, -1
-// when none; the longest row (0 without rows) in *longest, and CsrDev::reach
-// in *reach.
+// when none; the longest row (0 without rows) in *longest, and what a CsrDev
+// records of its rows (max_row, reach, wide_thr, wide_above) in *facts.
 std::pair<int64_t, int64_t> check_compressed(int32_t rows, int32_t cols, int64_t nnz,
                                              const int32_t *ptr, const int32_t *idx,
                                              cudaStream_t s, int32_t *longest = nullptr,
-                                             std::vector<int32_t> *reach = nullptr);
+                                             CsrDev *facts = nullptr);
 // COO (0-based device arrays, any order, duplicates allowed) -> CSR sorted by
 // (row, column), duplicates kept in input order. Returns -1, or the first
 // entry whose row or column is out of range (then `out` is untouched).
@@ -700,9 +706,10 @@ int64_t coo_to_csr(int32_t m, int32_t n, int64_t nnz, const int32_t *row, const 
                    const void *vals, Vt vt, CsrDev &out, cudaStream_t s);
 void csr_to_bsr(const CsrDev &c, int32_t m, int32_t n, int bs, int layout,
                 BsrDev &out, cudaStream_t s);
-// Rows of more than `threshold` entries, longest first, and their lengths.
-void list_long_rows(const DevBuf &row_ptr, int32_t m, int threshold, DevBuf &rows,
-                    std::vector<int32_t> &lens, cudaStream_t s);
+// The columns' memory (c.nnz of them), with room for the list of wide rows.
+void csr_reserve_columns(CsrDev &c, int32_t m);
+// CsrDev::wide_list of a checked matrix.
+void csr_list_wide_rows(CsrDev &c, int32_t m, cudaStream_t s);
 void csr_build_long_rows(CsrDev &c, int32_t m, int threshold, cudaStream_t s);
 
 // Norms (double accumulate on device, result to host).

@@ -22,7 +22,7 @@
 namespace pls {
 
 // What a row-group launch computes beside the row groups: the n wide rows
-// (longer than `skip`, listed longest first), `tiles` column tiles each, take
+// (longer than `skip`, listed longer ones first), `tiles` column tiles each, take
 // the first n * tiles CTAs.
 struct WideRows {
   const int32_t *rows;
@@ -93,29 +93,6 @@ static bool rows_off32_fits(const CsrDev &c, int32_t m, int64_t ldb, int64_t ldc
   return c.ncols > 0 && (int64_t)c.ncols * ldb < INT32_MAX && (int64_t)m * ldc < INT32_MAX;
 }
 
-// Lists the rows far longer than the mean (more than 8 times it, and 128
-// entries), longest first, on the first SpMM of a matrix that has any. Under
-// stream capture nothing is built and they run as any other row.
-constexpr int kWideRow = 128;
-constexpr int kWideMean = 8;
-
-static void find_wide_rows(CsrDev &c, int32_t m, cudaStream_t s) {
-  if (c.wide_found || m <= 0)
-    return;
-  const int32_t thr =
-      (int32_t)std::max<double>(kWideRow, kWideMean * std::ceil((double)c.nnz / m));
-  if (c.max_row <= thr) {
-    c.wide_found = true;
-    return;
-  }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  PLS_CUDA(cudaStreamIsCapturing(s, &cap));
-  if (cap != cudaStreamCaptureStatusNone)
-    return;
-  list_long_rows(c.row_ptr, m, thr, c.wide_rows, c.wide_len, s);
-  c.wide_found = true;
-}
-
 // Whether the shared-entries mode applies to this lane shape: one lane group
 // per row (TN = 1) of at least 4 lanes, so a shared load covers a group of
 // U = 4 entries.
@@ -130,12 +107,12 @@ static bool launch_spmm_csr(const CsrDev &c, int32_t m, const X *B, int64_t ldb,
   // Wide rows: those with entries for every group of a CTA; shorter ones
   // would leave part of it idle.
   WideRows w{nullptr, 0, INT32_MAX, 1};
-  if (!c.wide_len.empty()) {
-    w.rows = c.wide_rows.as<int32_t>();
-    w.skip = std::max(c.wide_len.back() - 1, kSpmmInFlight * (256 >> sh.lg_tk));
-    w.n = (int32_t)(std::partition_point(c.wide_len.begin(), c.wide_len.end(),
-                                         [&](int32_t l) { return l > w.skip; }) -
-                    c.wide_len.begin());
+  if (c.n_wide() > 0) {
+    const int lg = 10 - sh.lg_tk;  // 2^lg entries: kSpmmInFlight for each of 256 >> lg_tk groups
+    static_assert(kSpmmInFlight == 4, "2^(2 + 8 - lg_tk)");
+    w.rows = c.wide_list;
+    w.skip = std::max(c.wide_thr, 1 << lg);
+    w.n = w.skip > c.wide_thr ? c.wide_above[lg] : c.n_wide();
     w.tiles = (int32_t)div_up(k, (int64_t)VEC << sh.lg_tk);
   }
   const unsigned blocks = (unsigned)(div_up(m, rows_per_block) + (int64_t)w.n * w.tiles);
@@ -195,9 +172,8 @@ static int rows_vec(const CsrDev &c, int32_t m, const X *B, int64_t ldb, const X
 // arithmetic when `off32` and the offsets fit, and shared entry loads when
 // `shared` and the lane shape allows them (returns whether they ran).
 template <class X>
-static bool spmm_rows(CsrDev &c, int32_t m, const X *B, int64_t ldb, X *C, int64_t ldc,
+static bool spmm_rows(const CsrDev &c, int32_t m, const X *B, int64_t ldb, X *C, int64_t ldc,
                       int k, X alpha, X beta, bool off32, bool shared, cudaStream_t s) {
-  find_wide_rows(c, m, s);
   const int vec = rows_vec<X>(c, m, B, ldb, C, ldc, k, shared);
   bool ran = false;
   with_vt(c.evt(), [&](auto tag) {

@@ -683,3 +683,73 @@ def test_pageable_vectors_are_banded_by_size_alone(grid):
         used.append(A.host_bands_used())
     assert used[0] == m * 8 // 2 ** 20 if m * 8 < 2 ** 23 else used[0] == 8
     assert used[1:] == [m * 8 // 2 ** 22 if m * 8 >= 2 ** 23 else 0] * 3
+
+
+@pytest.mark.parametrize("create", ["csr", "coo", "csc"])
+def test_first_spmm_takes_no_longer_than_later_ones(create):
+    """The rows that get a CTA of their own are known from the creation: the
+    first product (row kernel forced, nothing timed) copies nothing to the host
+    and takes the time of a later one and some launches (it took 10 times as
+    long with 2 M power-law rows)."""
+    import time
+
+    import torch
+
+    m, n, rp, c, v = W.zipf_rows(2_000_000, seed=1)
+    k = 8
+    B = torch.rand((n, k), dtype=torch.float64, device="cuda")
+    C = torch.empty((m, k), dtype=torch.float64, device="cuda")
+
+    def handle():
+        if create == "csr":
+            A = pls.SpMat.csr(m, n, rp, c, v)
+        elif create == "coo":
+            A = pls.SpMat.coo(m, n, np.repeat(np.arange(m, dtype=np.int32), np.diff(rp)), c, v)
+        else:
+            order = np.argsort(c, kind="stable")
+            cp = np.zeros(n + 1, np.int32)
+            cp[1:] = np.cumsum(np.bincount(c, minlength=n))
+            A = pls.SpMat.csc(m, n, np.repeat(np.arange(m, dtype=np.int32), np.diff(rp))[order], cp, v[order])
+        A.set_spmm_path(0)
+        return A
+
+    def seconds(A):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        A.spmm_dev(B.data_ptr(), k, k, C.data_ptr(), k)
+        torch.cuda.synchronize()
+        return time.perf_counter() - t
+
+    first, later = [], []
+    for _ in range(3):  # the first handle's first call loads the kernels
+        A = handle()
+        first.append(seconds(A))
+        later += [seconds(A) for _ in range(3)]
+        A.destroy()
+    assert min(first[1:]) <= 1.5 * min(later) + 3e-4, (first, later)
+
+
+@pytest.mark.parametrize("create", ["csr", "coo", "csc", "trans"])
+def test_spmm_wide_rows_of_every_creation_path(create):
+    """The listed rows in the order of their lengths, equal ones among them, the
+    first and the last row of the matrix too."""
+    import torch
+
+    rng = np.random.default_rng(4)
+    n, k = 2500, 16
+    rp, c, v = csr_of_lengths([900] + [3] * 500 + [700, 129, 128, 900, 2000] + [4] * 400 + [900], n, rng)
+    m = len(rp) - 1
+    rows = np.repeat(np.arange(m, dtype=np.int32), np.diff(rp))
+    order = np.lexsort((rows, c))
+    cp = np.zeros(n + 1, np.int32)
+    cp[1:] = np.cumsum(np.bincount(c, minlength=n))
+    B = rng.uniform(-1, 1, (n, k))
+    Bm, C0 = pls.SpMat.dense(pls.ROW_MAJOR, n, k, k, B), pls.SpMat.dense(pls.ROW_MAJOR, m, k, k, np.zeros((m, k)))
+    if create == "trans":  # of A^T, whose columns are the wide rows
+        A, op = pls.SpMat.csr(n, m, cp, rows[order], v[order]), pls.OPERATION_TRANS
+    else:
+        A = {"csr": lambda: pls.SpMat.csr(m, n, rp, c, v), "coo": lambda: pls.SpMat.coo(m, n, rows, c, v),
+             "csc": lambda: pls.SpMat.csc(m, n, rows[order], cp, v[order])}[create]()
+        op = pls.OPERATION_NOTRANS
+    pls.spmm_exec(op, pls.OPERATION_NOTRANS, 1.0, A, Bm, 0.0, C0)
+    check(C0.export_dense(), oracle.csr_spmm(rp, c, v, B, k), oracle.csr_spmm(rp, c, np.abs(v), np.abs(B), k), 1e-12)

@@ -22,7 +22,13 @@ extern "C" {
 
 /* ---- device-pointer execution ----------------------------------------
  * Same semantics as perflibs_spmv_exec_{s,d} (y = alpha*op(A)*x + beta*y),
- * on device arrays, without host copies or synchronisation. */
+ * on device arrays, without host copies or synchronisation.
+ *
+ * Products of one handle that overlap on the GPU (two streams): a handle whose
+ * SELL layout has sliced chunks (n_split > 0 of perflibs_b200_spmat_exec_info:
+ * some rows far longer than the rest) keeps the slices' partial sums and counts,
+ * and overlapping products race on them; order them with events, or use a
+ * handle per stream. */
 perflibs_status_t perflibs_b200_spmv_exec_d_dev(
     enum perflibs_sparse_hint_value trans, double alpha, perflibs_spmat_t A,
     const double *x, double beta, double *y, void *stream);

@@ -753,3 +753,33 @@ def test_spmm_wide_rows_of_every_creation_path(create):
         op = pls.OPERATION_NOTRANS
     pls.spmm_exec(op, pls.OPERATION_NOTRANS, 1.0, A, Bm, 0.0, C0)
     check(C0.export_dense(), oracle.csr_spmm(rp, c, v, B, k), oracle.csr_spmm(rp, c, np.abs(v), np.abs(B), k), 1e-12)
+
+
+@pytest.mark.parametrize("C_,sigma", [(8, 0), (16, 1024), (32, 8192)])
+@pytest.mark.parametrize("wide", [129, 200, 256, 257, 600])
+def test_sell_layouts_without_much_to_slice_keep_no_partial_sums(wide, C_, sigma):
+    """Chunks of up to 256 columns among narrow ones are not sliced, so products
+    of one handle on two streams share nothing; wider ones are."""
+    import torch
+
+    rng = np.random.default_rng(wide)
+    m = 30_000
+    lens = np.where(np.arange(m) % 5000 == 77, wide, 1 + np.arange(m) % 3)
+    rp, c, v = csr_of_lengths(lens, m, rng)
+    A = pls.SpMat.csr(m, m, rp, c, v)
+    assert A.force_config(pls.KIND_SELL, C_, sigma, 0) == 0 and A.optimize() == 0
+    assert (A.exec_info()["n_split"] > 0) == (wide > 256)
+    if wide > 256:
+        return
+    xs = [torch.tensor(W.uniform_vector(m, i), device="cuda") for i in range(2)]
+    refs = [(oracle.csr_spmv(rp, c, v, x.cpu().numpy()), oracle.csr_absdot(rp, c, v, x.cpu().numpy())) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    ys = [torch.empty((20, m), dtype=torch.float64, device="cuda") for _ in xs]
+    torch.cuda.synchronize()
+    for i in range(20):
+        for x, y, st in zip(xs, ys, streams):
+            A.spmv_dev(x.data_ptr(), y[i].data_ptr(), stream=st.cuda_stream)
+    torch.cuda.synchronize()
+    for y, (ref, scale) in zip(ys, refs):
+        for i in (0, 7, 19):
+            check(y[i].cpu().numpy(), ref, scale, 1e-12)

@@ -142,7 +142,10 @@ inline cudaError_t launch_chained(void (*kern)(P...), unsigned grid, unsigned bl
   c.stream = s;
   c.attrs = &at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess)
+    cudaGetLastError();  // reported here, not by the next call's launch check
+  return e;
 }
 
 // Gathered elements of x (its pointer from chain_wait): plain loads, kept in

@@ -1,7 +1,7 @@
 // Autotune cache: checkpoint / resume for the exhaustive tuner.
 //
-// Every exhaustive tune is recorded under a key made of the GPU model, the
-// matrix's dimensions and nonzero count, the API and storage value types,
+// Every exhaustive tune is recorded under a key made of the GPU model and the
+// generation of the kernels (kKernels), the matrix's dimensions and nonzero count, the API and storage value types,
 // and a 64-bit hash of its sparsity structure (row pointers and column
 // indices; values do not change a kernel's speed). A later exhaustive
 // optimize with the same key takes the recorded configuration and timing
@@ -66,12 +66,19 @@ uint64_t structure_hash(const CsrDev &c, int32_t m, cudaStream_t s) {
   return h;
 }
 
+// Generation of the SpMV kernels and layouts that the candidates are timed with.
+// Raised whenever a change to them can change which candidate wins: entries of
+// another generation, from an older file, are then never found, and the matrix
+// is timed anew.
+constexpr int kKernels = 3;
+
 std::string device_signature(int dev) {
   int major = 0, minor = 0, sms = 0;
   PLS_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
   PLS_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
   PLS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  return "cc" + std::to_string(major) + std::to_string(minor) + "-sm" + std::to_string(sms);
+  return "cc" + std::to_string(major) + std::to_string(minor) + "-sm" + std::to_string(sms) +
+         "-k" + std::to_string(kKernels);
 }
 
 struct Entry {

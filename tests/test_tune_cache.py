@@ -64,3 +64,28 @@ def test_missing_file(tmp_path):
     with pytest.raises(pls.PerflibsError):
         pls.tune_cache_load(tmp_path / "absent.cache")
     assert pls.tune_cache_size() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("key", ["", "-k1"])
+def test_entries_of_other_kernels_are_timed_anew(tmp_path, key):
+    """A saved entry whose key names no generation of the kernels, or another
+    one, loads but is not taken."""
+    import re
+
+    from perf_libs_sparse_b200 import workloads as W
+
+    mat = W.zipf_rows(20_000, seed=5)
+    A = pls.SpMat.csr(*mat)
+    assert A.optimize() == 0 and A.tune_source() == pls.TUNE_SOURCE_TIMED
+    path = tmp_path / "now.cache"
+    pls.tune_cache_save(path)
+    old = tmp_path / "old.cache"
+    old.write_text(re.sub(r"^(cc\d+-sm\d+)(-k\d+)?", r"\1" + key, path.read_text(), flags=re.M))
+    for file, source in ((old, pls.TUNE_SOURCE_TIMED), (path, pls.TUNE_SOURCE_CACHE)):
+        pls.tune_cache_clear()
+        pls.tune_cache_load(file)
+        assert pls.tune_cache_size() == 1
+        B = pls.SpMat.csr(*mat)
+        assert B.optimize() == 0
+        assert B.tune_source() == source

@@ -204,13 +204,6 @@ template <int W, class T> __device__ __forceinline__ T group_sum(T v, unsigned m
   return v;
 }
 
-template <int W> __device__ __forceinline__ unsigned group_mask() {
-  if constexpr (W >= 32)
-    return 0xffffffffu;
-  else
-    return ((1u << W) - 1u) << ((threadIdx.x & 31) & ~(W - 1));
-}
-
 __host__ __device__ constexpr int64_t div_up(int64_t a, int64_t b) {
   return (a + b - 1) / b;
 }

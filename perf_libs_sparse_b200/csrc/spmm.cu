@@ -29,7 +29,7 @@ struct WideRows {
   int32_t n, skip, tiles;
 };
 
-template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES, bool WIDE>
+template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES, bool WIDE, bool KEEP_C>
 __device__ __forceinline__ void spmm_csr_rows(int32_t m, int lg_tk, int lg_tn, const WideRows &w,
                                               const int32_t *__restrict__ rp,
                                               const int32_t *__restrict__ col,
@@ -55,18 +55,18 @@ __device__ __forceinline__ void spmm_csr_rows(int32_t m, int lg_tk, int lg_tn, c
   const int lg_g = lg_tk + lg_tn;
   const int64_t warp = (block * blockDim.x + threadIdx.x) >> 5;
   const int64_t row = (warp << (5 - lg_g)) + ((threadIdx.x & 31) >> lg_g);
-  spmm_row_group<VEC, NV, Acc, X, CsrRows<V, WIDE>, OFF32, ENTRIES>(
+  spmm_row_group<VEC, NV, Acc, X, CsrRows<V, WIDE>, OFF32, ENTRIES, KEEP_C>(
       A, row, row < m, lg_tk, lg_tn, B, ldb, C, ldc, k, alpha, beta, beta_nz, pol);
 }
 
-template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES, bool WIDE>
+template <int VEC, int NV, class V, class X, bool OFF32, int ENTRIES, bool WIDE, bool KEEP_C>
 __global__ void __launch_bounds__(256)
     k_spmm_csr(int32_t m, int lg_tk, int lg_tn, WideRows w, const int32_t *__restrict__ rp,
                const int32_t *__restrict__ col, const V *__restrict__ val,
                const X *__restrict__ B, int64_t ldb, X *__restrict__ C, int64_t ldc, int k,
                X alpha, X beta, int beta_nz) {
-  spmm_csr_rows<VEC, NV, V, X, OFF32, ENTRIES, WIDE>(m, lg_tk, lg_tn, w, rp, col, val, B, ldb, C,
-                                                     ldc, k, alpha, beta, beta_nz);
+  spmm_csr_rows<VEC, NV, V, X, OFF32, ENTRIES, WIDE, KEEP_C>(m, lg_tk, lg_tn, w, rp, col, val, B,
+                                                             ldb, C, ldc, k, alpha, beta, beta_nz);
 }
 
 // Shared entries for FP32 results with one vector per lane, held to 48
@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(256, 5)
                       const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                       const V *__restrict__ val, const X *__restrict__ B, int64_t ldb,
                       X *__restrict__ C, int64_t ldc, int k, X alpha, X beta, int beta_nz) {
-  spmm_csr_rows<VEC, 1, V, X, OFF32, kEntriesShared, WIDE>(m, lg_tk, lg_tn, w, rp, col, val, B,
-                                                           ldb, C, ldc, k, alpha, beta, beta_nz);
+  spmm_csr_rows<VEC, 1, V, X, OFF32, kEntriesShared, WIDE, false>(
+      m, lg_tk, lg_tn, w, rp, col, val, B, ldb, C, ldc, k, alpha, beta, beta_nz);
 }
 
 // 32-bit address arithmetic is possible when every offset into B (rows
@@ -91,6 +91,19 @@ __global__ void __launch_bounds__(256, 5)
 // column count was not recorded.
 static bool rows_off32_fits(const CsrDev &c, int32_t m, int64_t ldb, int64_t ldc) {
   return c.ncols > 0 && (int64_t)c.ncols * ldb < INT32_MAX && (int64_t)m * ldc < INT32_MAX;
+}
+
+// Whether an FP32 C is stored to stay in L2 instead of leaving first: where
+// entries, B and C take up to half of it, C stays there anyway, and rows that
+// leave early are written to memory twice as soon. Leaving first against staying
+// (FP32, us): 60,000 x 18, k = 32 (24 MB) 22.5 / 21.4, 300,000 x 4, k = 8 and 16
+// (29 and 48 MB) 15.1 / 13.3 and 21.2 / 19.5, k = 32 (86 MB) 35.6 / 37.6,
+// 300,000 x 18, k = 16 (81 MB) 58.9 / 58.3, k = 32 (120 MB) 83 / 90. FP64
+// gains from 18 MB on (60,000 x 18, k = 32, 44 MB: 33.6 / 35.6).
+template <class X> static bool spmm_keeps_c(const CsrDev &c, int32_t m, int k) {
+  const int64_t bytes =
+      c.nnz * (int64_t)(vt_size(c.evt()) + 4) + ((int64_t)c.ncols + m) * k * (int64_t)sizeof(X);
+  return sizeof(X) == 4 && bytes <= (64 << 20);
 }
 
 // Whether the shared-entries mode applies to this lane shape: one lane group
@@ -117,18 +130,23 @@ static bool launch_spmm_csr(const CsrDev &c, int32_t m, const X *B, int64_t ldb,
   }
   const unsigned blocks = (unsigned)(div_up(m, rows_per_block) + (int64_t)w.n * w.tiles);
   const int bnz = beta != X(0);
+  const bool keep_c = spmm_keeps_c<X>(c, m, k);
   off32 = off32 && rows_off32_fits(c, m, ldb, ldc);
   shared = shared && shared_entries_fit(sh);
   auto go = [&](auto nv_tag, auto off_tag, auto entries_tag) {
     constexpr int NV = decltype(nv_tag)::value;
     constexpr bool OFF = decltype(off_tag)::value;
     constexpr int EM = decltype(entries_tag)::value;
-    auto kern = k_spmm_csr<VEC, NV, V, X, OFF, EM, false>;
+    auto kern = k_spmm_csr<VEC, NV, V, X, OFF, EM, false, false>;
     if constexpr (EM == kEntriesShared && NV == 1 && sizeof(X) == 4)
       kern = w.n > 0 ? k_spmm_csr_shared<VEC, V, X, OFF, true>
                      : k_spmm_csr_shared<VEC, V, X, OFF, false>;
     else if (w.n > 0)
-      kern = k_spmm_csr<VEC, NV, V, X, OFF, EM, true>;
+      kern = k_spmm_csr<VEC, NV, V, X, OFF, EM, true, false>;
+    if constexpr (EM == kEntriesLane && sizeof(X) == 4)
+      if (keep_c)
+        kern = w.n > 0 ? k_spmm_csr<VEC, NV, V, X, OFF, EM, true, true>
+                       : k_spmm_csr<VEC, NV, V, X, OFF, EM, false, true>;
     kern<<<blocks, 256, 0, s>>>(m, sh.lg_tk, sh.lg_tn, w, c.row_ptr.as<int32_t>(),
                                 c.col.as<int32_t>(), (const V *)c.ev(), B, ldb, C, ldc, k, alpha,
                                 beta, bnz);

@@ -49,10 +49,11 @@ __device__ __forceinline__ void ld_vec(const X *p, X (&v)[VEC]) {
 // again, are kept (evict last), and rows of C, which nothing here reads
 // again, are stored to leave first, so that C and the entries do not push B out
 // of L2 where the three together exceed it. Measured on random rows (old ->
-// new): 200,003 x 18, k = 64 FP32 108 -> 102 us, k = 32 FP64 119 -> 104 us, power
+// new): 200,003 x 18, k = 64 FP32 116 -> 111 us, k = 32 FP64 119 -> 104 us, power
 // law 400,003, k = 24 FP64 448 -> 385 us; 27-point stencil 95^3, k = 33 FP64
 // 896 -> 871 us, 5-point Laplacian 700^2, k = 9 FP64 81 -> 73 us; random 60,003 x
-// 18 (all in L2) 33 -> 33 us.
+// 18 (all in L2) 33 -> 33 us. Where the three are small, an FP32 C is stored
+// plainly (KEEP_C): see spmm_keeps_c.
 template <int VEC>
 __device__ __forceinline__ void ld_vec(const float *p, float (&v)[VEC], uint64_t pol) {
   if constexpr (VEC == 1)
@@ -171,9 +172,9 @@ constexpr int kEntriesLane = 0, kEntriesAhead = 1, kEntriesShared = 2;
 // pass live = false and only take part in the shuffles. TK, TN (as log2)
 // and k are uniform across the warp.
 // OFF32: every offset into B and C (row * ld + column) fits in 32 bits, so
-// the address arithmetic stays 32-bit.
+// the address arithmetic stays 32-bit. KEEP_C: C is stored to stay in L2.
 template <int VEC, int NV, class Acc, class X, class Rows, bool OFF32 = false,
-          int ENTRIES = kEntriesLane>
+          int ENTRIES = kEntriesLane, bool KEEP_C = false>
 __device__ __forceinline__ void spmm_row_group(const Rows &A, int64_t row, bool live, int lg_tk,
                                                int lg_tn, const X *__restrict__ B, int64_t ldb,
                                                X *__restrict__ C, int64_t ldc, int k, X alpha,
@@ -318,7 +319,7 @@ __device__ __forceinline__ void spmm_row_group(const Rows &A, int64_t row, bool 
             for (int v = 0; v < VEC; ++v)
               out[v] = (X)acc[nv][v] * alpha;
           }
-          if constexpr (ENTRIES == kEntriesShared)
+          if constexpr (ENTRIES == kEntriesShared || KEEP_C)
             st_vec<X, VEC>(crow + kk, out);
           else
             st_vec_stream<X, VEC>(crow + kk, out);

@@ -783,3 +783,34 @@ def test_sell_layouts_without_much_to_slice_keep_no_partial_sums(wide, C_, sigma
     for y, (ref, scale) in zip(ys, refs):
         for i in (0, 7, 19):
             check(y[i].cpu().numpy(), ref, scale, 1e-12)
+
+
+@pytest.mark.parametrize("k", [80, 81, 82, 88])
+@pytest.mark.parametrize("wide", [False, True])
+def test_spmm_fp32_on_both_sides_of_the_store_rule(k, wide):
+    """Entries, B and C just below and above the 64 MB up to which C is stored to
+    stay in L2, in whole vectors and column by column, with beta."""
+    import torch
+
+    rng = np.random.default_rng(k)
+    m = 100_000
+    lens = 1 + np.arange(m) % 5
+    if wide:
+        lens[::40_000] = 700
+    rp = np.zeros(m + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    c = rng.integers(0, m, int(rp[-1])).astype(np.int32)
+    v = rng.uniform(-1, 1, len(c)).astype(np.float32)
+    total = len(c) * 8 + 2 * m * k * 4
+    assert (total <= 64 * 2 ** 20) == (k <= 80)
+    A = pls.SpMat.csr(m, m, rp, c, v)
+    A.set_spmm_path(0)
+    B, C0 = rng.uniform(-1, 1, (m, k)).astype(np.float32), rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    Bd, Cd = torch.tensor(B, device="cuda"), torch.tensor(C0, device="cuda")
+    torch.cuda.synchronize()
+    A.spmm_dev(Bd.data_ptr(), k, k, Cd.data_ptr(), k, 1.5, -0.5)
+    torch.cuda.synchronize()
+    v64, B64 = v.astype(np.float64), B.astype(np.float64)
+    ref = 1.5 * oracle.csr_spmm(rp, c, v64, B64, k) - 0.5 * C0
+    scale = 1.5 * oracle.csr_spmm(rp, c, np.abs(v64), np.abs(B64), k) + 0.5 * np.abs(C0)
+    check(Cd.cpu().numpy(), ref, scale, 1e-5)

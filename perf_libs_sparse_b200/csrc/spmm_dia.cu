@@ -563,10 +563,21 @@ void dia_launch(const CsrDev &c, int32_t m, const X *B, int64_t ldb, X *C, int64
   const DiaPatchPlan patch = dia_patch_plan(runs, kDiaRows, nunits, lg_tk);
   const unsigned grid = (unsigned)div_up(threads, 256);
   // Staging pays from 8 lanes per unit on, where the direct kernel loads each
-  // value in every lane: staged against direct, FP64 96^3 k = 16 (8 lanes)
-  // 134 / 168 us, FP32 128^3 k = 32 (8 lanes) 240 / 256 us; FP64 128^3 k = 8
-  // (4 lanes) 231 / 230 us, FP32 k = 8 (2 lanes) 176 / 157 us.
-  if (lg_tk < 3) {
+  // value in every lane, and from so many runs on that there are values enough
+  // to load (5 for an FP32 B, 3 for an FP64 B with narrower values, 2 with FP64
+  // ones); not for BF16 values in 8 lanes where the runs lie far apart.
+  // Staged / direct (us): FP64 96^3 k = 16 (8 lanes) 134 / 168,
+  // 128^3 k = 8 (4 lanes) 231 / 230; FP32 128^3 k = 32 (8 lanes) 240 / 256, k = 8
+  // (2 lanes) 176 / 157. Bands of 3 (one run), 600,000 rows: FP32 k = 128 112 / 96,
+  // FP64 k = 64 112 / 109; of 5 (2 runs): FP32 k = 64 64 / 58, FP64 with BF16
+  // values k = 32 63 / 58, FP64 k = 32 64 / 71; 5-point Laplacian 800^2 (3 runs):
+  // FP32 k = 128 144 / 134, FP64 with BF16 values k = 32 77 / 83; bands of 15 (5
+  // runs), 400,000 rows, FP32 k = 64 60 / 64. BF16, 8 lanes: stencil 110^3
+  // 155 / 151, 128^3 237 / 235, 64^3 35.5 / 36.2, band of 31 54 / 63.
+  const int min_runs = sizeof(X) == 4 ? 5 : sizeof(V) == 8 ? 2 : 3;
+  const bool far_runs = (int64_t)d.offs[d.nd - 1] - d.offs[0] > 16384;
+  if (lg_tk < 3 || runs.n < min_runs ||
+      (sizeof(V) == 2 && sizeof(X) == 4 && lg_tk == 3 && far_runs)) {
     k_spmm_dia<V, X, VEC><<<grid, 256, 0, s>>>(m, c.ncols, d.nd, runs, d.vals.as<V>(), B, ldb, C,
                                                ldc, k, lg_tk, patch, alpha, beta, beta != X(0));
   } else {

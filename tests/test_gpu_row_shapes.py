@@ -239,6 +239,19 @@ def dia_matrix(name, rng):
         return W.laplacian_2d(23)
     if name == "lines":  # lines of 64 rows: line patches
         return stencil_2d9(64, 40, rng)
+    if name == "band1":  # one run
+        return W.banded_csr(299, 1, rng)
+    if name == "band2":  # two runs
+        return W.banded_csr(301, 2, rng)
+    if name == "band7":  # five runs
+        return W.banded_csr(302, 7, rng)
+    if name == "far5":  # five runs, more than 16384 rows apart
+        i = np.arange(40_000)
+        cols = i[:, None] + np.array([-18_000, -200, 0, 200, 18_000])
+        ok = (cols >= 0) & (cols < 40_000)
+        rp = np.zeros(40_001, np.int32)
+        rp[1:] = np.cumsum(ok.sum(1))
+        return 40_000, 40_000, rp, cols[ok].astype(np.int32), rng.standard_normal(int(rp[-1]))
     if name == "band15":  # 31 consecutive diagonals: the last run is one diagonal
         return W.banded_csr(301, 15, rng)
     m, n = (260, 400) if name == "wide" else (403, 250)  # a band in a matrix that is not square
@@ -250,7 +263,8 @@ def dia_matrix(name, rng):
     return m, n, rp, c[keep].astype(np.int32), rng.standard_normal(int(rp[-1]))
 
 
-@pytest.mark.parametrize("name", ["stencil27", "laplace", "lines", "band15", "wide", "tall"])
+@pytest.mark.parametrize("name", ["stencil27", "laplace", "lines", "band15", "wide", "tall", "band1", "band2", "band7",
+                                  "far5"])
 @pytest.mark.parametrize("dtype,storage", [(np.float64, "native"), (np.float64, "fp32"), (np.float64, "bf16"),
                                            (np.float32, "native"), (np.float32, "bf16")])
 def test_diagonal_form_equals_row_kernel_at_every_lane_count(name, dtype, storage):
@@ -293,13 +307,14 @@ def test_diagonal_form_equals_row_kernel_at_every_lane_count(name, dtype, storag
                 np.testing.assert_allclose(out[0][fin], out[1][fin], rtol=tol, atol=tol)
 
 
-def test_diagonal_form_beyond_32_bit_offsets():
+@pytest.mark.parametrize("half_bandwidth", [1, 7])  # values read directly, staged values
+def test_diagonal_form_beyond_32_bit_offsets(half_bandwidth):
     """Rows of B and C 65,600 elements apart: offsets past 2^32 elements."""
     import torch
 
-    m, ld, k = 65_700, 65_600, 32  # staged values
+    m, ld, k = 65_700, 65_600, 32
     rng = np.random.default_rng(2)
-    _, _, rp, c, v = W.banded_csr(m, 1, rng)
+    _, _, rp, c, v = W.banded_csr(m, half_bandwidth, rng)
     A = pls.SpMat.csr(m, m, rp, c, v.astype(np.float32))
     A.set_spmm_path(3)
     B = torch.empty((m, ld), dtype=torch.float32, device="cuda")

@@ -77,8 +77,8 @@ inline DiaRuns dia_runs(const int32_t *offs, int nd) {
   return r;
 }
 
-// What the diagonal-form SpMM with staged values (k_spmm_dia_staged) walks: the runs in ascending
-// order, cut into chunks whose values it holds in shared memory at a time (as
+// What the diagonal-form SpMM with staged values (k_spmm_dia_staged) walks: the
+// runs in ascending order, cut into chunks whose values it holds in shared memory at a time (as
 // many whole runs as keep a 256-thread CTA's 256 / 2^lg_tk units within
 // kDiaSlabBytes: four CTAs share an SM and leave half of it to L1), and the
 // chunks into segments of runs of one length. A unit's slab is unit_bytes: its

@@ -19,7 +19,11 @@
 // It also replays the line-patch plan of the kernel that reads B through L1
 // (k_spmm_dia: dia_patch_plan / dia_patch_unit in the same header) over
 // every CTA and thread: every unit of rows is computed exactly once, and
-// each patch CTA holds whole line segments.
+// each patch CTA holds whole line segments. And the walk of the kernel that
+// stages a unit's values (k_spmm_dia_staged: dia_walk): chunks, segments and
+// runs cover every diagonal once in ascending order, copies and reads stay
+// inside a unit's slab and the diagonal form and are aligned, the slabs fit the
+// launch's shared memory, and every row of B used is the entry's own.
 // Prints "ok <cases>" or the first violation (exit status 1).
 #include <cstdio>
 #include <cstdlib>
@@ -309,6 +313,62 @@ static bool replay_patches(const Case &cs, int lg_tk, int rb) {
   return p.units > 0;
 }
 
+// k_spmm_dia_staged with 2^lg_tk lanes per unit, values of vb bytes and rows of
+// B ldb elements apart; the matrix has n columns. Returns the chunks.
+static int replay_walk(const Case &cs, int lg_tk, int vb, int64_t ldb, int32_t n) {
+  const char *nm = cs.name.c_str();
+  const int nd = (int)cs.offs.size(), piece = vb == 2 ? 8 : 16, diag_bytes = kDiaRows * vb;
+  const DiaRuns runs = dia_runs(cs.offs.data(), nd);
+  const DiaWalk w = dia_walk(runs, lg_tk, vb, ldb);
+  CHECK(w.n_chunks >= 1 && w.n_chunks <= kDiaMax, "%s chunks %d", nm, w.n_chunks);
+  CHECK(w.unit_bytes % 16 == 0 && w.unit_bytes / 16 % 2 == 1, "%s unit_bytes %d", nm, w.unit_bytes);
+  CHECK(((int64_t)w.unit_bytes << (8 - lg_tk)) <= kDiaSlabBytes, "%s slabs of %d bytes", nm, w.unit_bytes);
+  CHECK(w.seg0[0] == 0 && w.run0[0] == 0 && w.d0[0] == 0 && w.d0[w.n_chunks] == nd, "%s ends", nm);
+  CHECK(w.run0[w.seg0[w.n_chunks]] == runs.n, "%s every run", nm);
+  // The walk itself, the same for every unit: (diagonal, its place in the slab).
+  std::vector<int> place;
+  for (int c = 0; c < w.n_chunks; ++c) {
+    CHECK(w.d0[c + 1] > w.d0[c] && w.seg0[c + 1] > w.seg0[c], "%s empty chunk", nm);
+    CHECK((w.d0[c + 1] - w.d0[c]) * diag_bytes <= w.unit_bytes, "%s chunk %d fits", nm, c);
+    CHECK((w.d0[c + 1] - w.d0[c]) * diag_bytes % piece == 0, "%s whole pieces", nm);
+    int at = 0;  // diagonals of the chunk walked
+    for (int g = w.seg0[c]; g < w.seg0[c + 1]; ++g) {
+      CHECK(w.len[g] >= 1 && w.len[g] <= kDiaRun && w.run0[g + 1] > w.run0[g], "%s segment", nm);
+      for (int q = w.run0[g]; q < w.run0[g + 1]; ++q) {
+        CHECK(runs.len[q] == w.len[g] && runs.d0[q] == (int)place.size(), "%s run %d", nm, q);
+        CHECK(w.o0[q] == runs.o0[q] && w.at[q] == (int64_t)runs.o0[q] * ldb, "%s run %d", nm, q);
+        for (int l = 0; l < w.len[g]; ++l, ++at) {
+          CHECK(w.d0[c] + at == (int)place.size(), "%s ascending", nm);
+          CHECK(cs.offs[place.size()] == w.o0[q] + l, "%s offset of diagonal %zu", nm, place.size());
+          CHECK(at * diag_bytes % (diag_bytes < 16 ? 8 : 16) == 0, "%s read alignment", nm);
+          place.push_back(at);
+        }
+      }
+    }
+    CHECK(at == w.d0[c + 1] - w.d0[c], "%s chunk %d walked", nm, c);
+  }
+  CHECK((int)place.size() == nd, "%s every diagonal once", nm);
+  // Every unit's copies, and its rows of B through the offsets of the launch.
+  const int64_t dia_bytes = plan_div_up((int64_t)cs.m + kDiaPadRows, kDiaRows) * nd * diag_bytes + 16;
+  const bool off32 = ((int64_t)cs.m + 2 * kDiaRows + kDiaRun) * ldb < (int64_t)UINT32_MAX;
+  const int last = runs.n - 1;
+  for (int64_t u = 0; u * kDiaRows < cs.m; ++u) {
+    const int64_t r0 = u * kDiaRows;
+    CHECK((u + 1) * nd * diag_bytes <= dia_bytes && u * nd * diag_bytes % piece == 0, "%s unit copies", nm);
+    const bool inside =
+        r0 + w.o0[0] >= 0 && r0 + w.o0[last] + w.len[w.seg0[w.n_chunks] - 1] + kDiaRows - 2 < n;
+    for (int q = 0; q < runs.n; ++q)
+      for (int j = 0; j < kDiaRows + runs.len[q] - 1; ++j) {
+        const int64_t brow = r0 + w.o0[q] + j, at = (r0 + j) * ldb;
+        CHECK(!inside || (brow >= 0 && brow < n), "%s row %lld of an inside unit", nm, (long long)brow);
+        CHECK(!off32 || at + ldb - 1 <= (int64_t)UINT32_MAX, "%s 32-bit offset", nm);
+        CHECK(w.at[q] + at == brow * ldb, "%s address of row %lld", nm, (long long)brow);
+      }
+    // entry (row i, diagonal l of run q) uses bv[i + l], row r0 + o0 + i + l
+  }
+  return w.n_chunks;
+}
+
 int main() {
   std::vector<Case> cases = {
       {"27pt-128", 128 * 128 * 128, stencil3d(128, true), {8, 32, 128}},
@@ -366,7 +426,25 @@ int main() {
               plan_div_up(c3.m, kDiaRows),
           "C3 line patches, lg_tk=%d", lg_tk);
   }
-  std::printf("ok %d of %d configurations applied and replayed; line patches in %d of %d\n",
-              applied, tried, patched, ptried);
+  // Bands of up to kDiaMax diagonals, whose values take several chunks of a slab.
+  std::vector<Case> walks = cases;
+  walks.push_back({"band31", 301, band(-15, 15)});
+  walks.push_back({"band32", 400, band(-15, 16)});
+  walks.push_back({"band20", 402, band(-9, 10)});
+  walks.push_back({"far5", 40000, {-18000, -200, 0, 200, 18000}});
+  walks.push_back({"mixed", 260, {-40, -39, -7, -2, -1, 0, 1, 6, 30, 31, 32, 33, 34}});
+  int walked = 0, chunked = 0;
+  for (const Case &cs : walks)
+    for (int lg_tk = 3; lg_tk <= 5; ++lg_tk)
+      for (int vb : {8, 4, 2})
+        for (int64_t ldb : {int64_t(16), int64_t(65600)})
+          for (int32_t n : {cs.m, cs.m + 140, std::max(1, cs.m - 153)}) {
+            ++walked;
+            chunked += replay_walk(cs, lg_tk, vb, ldb, n) > 1 ? 1 : 0;
+          }
+  CHECK(chunked > 0, "no walk of several chunks");
+  std::printf("ok %d of %d configurations applied and replayed; line patches in %d of %d; walks of "
+              "several chunks %d of %d\n",
+              applied, tried, patched, ptried, chunked, walked);
   return 0;
 }

@@ -10,7 +10,9 @@ waited for once before its first read and never overwritten while read,
 every read must hit the B row its entry needs, and every element of C must
 be written exactly once. It also replays the line-patch assignment of the
 diagonal-form kernel that reads B through L1 (every unit of rows computed
-exactly once, for every lane count and both unit sizes)."""
+exactly once, for every lane count and both unit sizes), and the walk of the
+kernel that stages a unit's values (every diagonal once, every copy and read
+inside its slab, every row of B the entry's own)."""
 import os
 import shutil
 import subprocess

@@ -28,7 +28,15 @@ extern "C" {
  * SELL layout has sliced chunks (n_split > 0 of perflibs_b200_spmat_exec_info:
  * some rows far longer than the rest) keeps the slices' partial sums and counts,
  * and overlapping products race on them; order them with events, or use a
- * handle per stream. */
+ * handle per stream.
+ *
+ * The SpMV kernels are launched with programmatic stream serialisation: a
+ * product may be started while the kernel before it on the stream drains, and
+ * waits for it before it touches x or y. Stream order is as ever for the
+ * caller. A graph captured from such calls has programmatic edges: queries of
+ * its edges without edge data (cudaGraphGetEdges, cudaGraphNodeGetDependencies
+ * and the like in their older forms) return cudaErrorLossyQuery; use the
+ * forms that return cudaGraphEdgeData. */
 perflibs_status_t perflibs_b200_spmv_exec_d_dev(
     enum perflibs_sparse_hint_value trans, double alpha, perflibs_spmat_t A,
     const double *x, double beta, double *y, void *stream);

@@ -829,3 +829,110 @@ def test_spmm_fp32_on_both_sides_of_the_store_rule(k, wide):
     ref = 1.5 * oracle.csr_spmm(rp, c, v64, B64, k) - 0.5 * C0
     scale = 1.5 * oracle.csr_spmm(rp, c, np.abs(v64), np.abs(B64), k) + 0.5 * np.abs(C0)
     check(Cd.cpu().numpy(), ref, scale, 1e-5)
+
+
+def chained_handle(fmt, n, rng):
+    if fmt == "bsr4":
+        rp, c, _ = csr_of_lengths(np.full(n // 4, 3), n // 4, rng)
+        return pls.SpMat.bsr(pls.ROW_MAJOR, n, n, 4, rp, c, rng.uniform(-1, 1, len(c) * 16) / 8)
+    lens = rng.integers(0, 9, n)
+    lens[::1500] = 900
+    rp, c, v = csr_of_lengths(lens, n, rng)
+    A = pls.SpMat.csr(n, n, rp, c, v / 30)
+    A.force_config(*{"csr": (pls.KIND_CSR, 0, 0, 2), "sell": (pls.KIND_SELL, 16, 0, 0)}[fmt])
+    assert A.optimize() == 0
+    return A
+
+
+@pytest.mark.parametrize("fmt", ["csr", "sell", "bsr4"])
+def test_chained_products_after_copies_fills_and_joins(fmt):
+    """Captured products whose predecessor in the stream is a copy, a fill or a
+    join with another stream, replayed on new x: the bits of the same work with
+    a synchronisation after each step."""
+    import torch
+
+    rng = np.random.default_rng(8)
+    n = 4096
+    A = chained_handle(fmt, n, rng)
+    s, other = torch.cuda.Stream(), torch.cuda.Stream()
+    x, a, b, c = (torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(4))
+
+    def product(src, dst, alpha=1.0, beta=0.0):
+        A.spmv_dev(src.data_ptr(), dst.data_ptr(), alpha, beta, stream=s.cuda_stream)
+
+    def steps(sync):
+        def done():
+            if sync:
+                torch.cuda.synchronize()
+
+        for _ in range(6):
+            a.copy_(x)  # a copy
+            done()
+            product(a, b)
+            done()
+            c.zero_()  # a fill
+            done()
+            product(b, c, 1.0, 1.0)
+            done()
+            other.wait_stream(s)
+            with torch.cuda.stream(other):
+                a.add_(c)  # on another stream, joined
+            done()
+            s.wait_stream(other)
+            product(a, b, 0.5, 0.25)
+            done()
+            product(b, x)
+            done()
+
+    xs = [torch.tensor(W.uniform_vector(n, 20 + i), device="cuda") for i in range(3)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin(capture_error_mode="thread_local")
+        steps(False)
+        graph.capture_end()
+    for x0 in xs:
+        out = []
+        for mode in ("sync", "queued", "graph"):
+            for t in (a, b, c):
+                t.fill_(3.0)
+            x.copy_(x0)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(s):
+                graph.replay() if mode == "graph" else steps(mode == "sync")
+            torch.cuda.synchronize()
+            out.append([t.cpu().numpy() for t in (x, a, b, c)])
+        assert np.isfinite(out[0][0]).all() and np.abs(out[0][0]).max() > 0
+        for got in out[1:]:
+            for g, w in zip(got, out[0]):
+                np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("fmt", ["csr", "sell"])
+def test_chained_products_around_a_value_update(fmt):
+    """Products queued before and after an update of the handle's values: those
+    before use the old values, those after the new ones."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    n = 4096
+    s = torch.cuda.Stream()
+    x0 = torch.tensor(W.uniform_vector(n, 3), device="cuda")
+    out = []
+    for sync in (True, False):
+        A = chained_handle(fmt, n, np.random.default_rng(9))
+        _, _, rp, c, v = A.export_csr()
+        rows = np.repeat(np.arange(n, dtype=np.int32), np.diff(rp))
+        A.set_stream(s.cuda_stream)
+        ys = [torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(20)]
+        torch.cuda.synchronize()
+        for i, y in enumerate(ys):
+            if i == 10:
+                A.update(rows, c, 2.0 * v)
+            A.spmv_dev((ys[i - 1] if i else x0).data_ptr(), y.data_ptr(), stream=s.cuda_stream)
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        out.append(np.stack([y.cpu().numpy() for y in ys]))
+    assert np.isfinite(out[0]).all() and np.abs(out[0][-1]).max() > 0
+    np.testing.assert_array_equal(out[0], out[1])

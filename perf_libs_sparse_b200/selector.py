@@ -530,7 +530,8 @@ def evaluate(corpus, n_train: int, out_dir: str, epochs=400, batch=128, lr=3e-3,
     best = Th.min(1)
     chosen = Th[np.arange(len(Th)), cls]
     regret = chosen / best - 1.0
-    # plain FP64 CSR: the default kernel (threads per row = 2^floor(log2 mean))
+    # plain FP64 CSR: the CSR kernel with 2^floor(log2 mean) lanes per row (the
+    # corpus does not record the longest row, which the default lanes look at too)
     mean_len = nnz[n_train:] / np.maximum(m[n_train:], 1)
     tpr = np.clip(2 ** np.floor(np.log2(np.maximum(mean_len, 1))), 1, 32).astype(int)
     plain_idx = np.array([int(np.flatnonzero((cands[:, 0] == KIND_CSR) & (cands[:, 3] == t))[0]) for t in tpr])

@@ -74,7 +74,7 @@ struct Item {
 // A staged item: rows [row0, row1) of instance `inst`, whose entries all
 // have columns in [lo, lo + w), for C's columns [c0, c0 + ks) (ks <= 32).
 // The window sits in shared memory as w rows of 4 * tk floats (ks rounded
-// up to whole float4s, zero past ks).
+// up to whole float4s, zero past ks), 4 * stage_stride(tk) floats apart.
 struct SItem {
   int32_t inst, row0, row1, lo;
   int32_t w, c0, ks, tk;
@@ -235,12 +235,15 @@ __device__ __forceinline__ BandBlock band_block(const int2 *__restrict__ rng, in
 }
 
 // One staged item, by the whole CTA. The window of B (rows lo .. lo + w - 1,
-// columns c0 .. c0 + ks - 1) is copied into `stage` (row stride 4 tk
-// floats); then tk lanes per row own 4 columns each, and every row of the
-// item adds its entries in stored order from the staged rows. Each entry's
-// column lies in the window (the item was built from the minimum and
-// maximum column of its entries), so the stage reads stay inside
-// w * 4 tk floats.
+// columns c0 .. c0 + ks - 1) is copied into `stage` (row stride
+// 4 * stage_stride(tk) floats); then tk lanes per row own 4 columns each, and
+// every row of the item adds its entries in stored order from the staged rows.
+// Each entry's column lies in the window (the item was built from the minimum
+// and maximum column of its entries), so the stage reads stay inside
+// w * 4 * stage_stride(tk) floats. These fit kStageFloats: w is at most what the
+// instance's first, widest column slice leaves, and a narrower last slice has no
+// larger stride (only k > 32 has several slices, the first of 8 lanes and stride
+// 8, the last of at most 8 lanes and stride at most 8).
 __device__ __forceinline__ void staged_item(const SItem &w, const InstDesc &d,
                                             float *__restrict__ stage, float alpha, float beta,
                                             int beta_nz) {
@@ -699,8 +702,9 @@ void build_items(Batch *B, int32_t tile) {
 
 // The staged items, once at creation (the packed entries must be in
 // place). Each instance with k >= 1 is cut into blocks of rs rows, rs half
-// the window rows its widest column slice (min(k, 32) columns, rounded up
-// to float4s) leaves in kStageFloats. A block is staged when its entries'
+// the window rows that its widest column slice (min(k, 32) columns, rounded up
+// to float4s, at the stage's stride) leaves in kStageFloats, in whole blocks of
+// 4 rows for every lane group of a warp. A block is staged when its entries'
 // column window fits in the stage and holds at most half as many rows of B
 // as the block has entries (each staged B row read at least twice on
 // average); it then gives one item per column slice of 32. The other rows
@@ -728,7 +732,6 @@ void build_staged(Batch *B) {
     }
     const int32_t tk0 = stage_lanes(d.k);
     const int32_t wmax = kStageFloats / (4 * stage_stride(tk0));
-    // whole blocks of 4 rows for every lane group of a warp
     const int32_t rs = wmax / 2 / (4 * (32 / tk0)) * (4 * (32 / tk0));
     const int64_t nblk = div_up((int64_t)d.m, (int64_t)rs);
     win.reserve(sizeof(int4) * nblk);

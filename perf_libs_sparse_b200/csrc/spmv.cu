@@ -110,14 +110,19 @@ __device__ __forceinline__ Acc csr_lane_sum(uint32_t j, uint32_t e, const int32_
 //
 // chain_next after the sum, as in k_sell: 30,000 FP64 rows of 14 entries
 // 5.8 us with it first, 4.5 us after the sum, geometric lengths of mean 10 on 4
-// lanes 6.1 and 5.1; at 300,000 rows equal.
-template <int TPR, bool LONG, class V, class X>
+// lanes 6.1 and 5.1; equal at 300,000 rows on 4 lanes. First (EARLY) in grids
+// of many waves without the long-row part, whose CTAs even out: 300,000 rows of
+// 0 to 28 entries on 8 lanes 22.8 against 23.1 us, of 40 on 16 lanes 56.1 / 56.7.
+constexpr int64_t kCsrEarlyCtas = 148 * 8 * 6;
+template <int TPR, bool LONG, bool EARLY, class V, class X>
 __global__ void __launch_bounds__(256)
     k_csr_vector(int32_t m, const int32_t *__restrict__ rp,
                  const int32_t *__restrict__ col, const V *__restrict__ val,
                  const X *xg, X *y, X alpha, X beta, int beta_nz, int32_t skip_len) {
   using Acc = typename AccOf<V, X>::type;
   constexpr int G = csr_group(TPR);
+  if constexpr (EARLY)
+    chain_next();
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t row = gid / TPR;
   const int sub = threadIdx.x & (TPR - 1);
@@ -149,7 +154,8 @@ __global__ void __launch_bounds__(256)
         sum = t;
     }
   }
-  chain_next();
+  if constexpr (!EARLY)
+    chain_next();
   if (sub == 0 && live)
     store_y(y, row, sum, alpha, beta, beta_nz);
 }
@@ -190,10 +196,11 @@ static void launch_csr_vector(const CsrDev &c, int64_t r0, int32_t m, const X *x
   const int64_t blocks = div_up(threads, 256);
   // The long-row kernel beside this one (skip) takes the long rows itself.
   const bool has_long = skip == 0 && c.max_row > csr_long_len(TPR);
-  auto kern = k_csr_vector<TPR, false, V, X>;
+  auto kern = blocks >= kCsrEarlyCtas ? k_csr_vector<TPR, false, true, V, X>
+                                      : k_csr_vector<TPR, false, false, V, X>;
   if constexpr (TPR < 32)
     if (has_long)
-      kern = k_csr_vector<TPR, true, V, X>;
+      kern = k_csr_vector<TPR, true, false, V, X>;
   PLS_CUDA(launch_chained(kern, (unsigned)blocks, 256, s, m, c.row_ptr.as<int32_t>() + r0,
                           c.col.as<int32_t>(), (const V *)c.ev(), x, y + r0, alpha, beta,
                           beta != X(0), skip));

@@ -465,8 +465,9 @@ __device__ __forceinline__ void ld_block_line(const V *p, V (&a)[BS]) {
 // Bound by the latency of B's rows. Blocks of 8 are held to two CTAs per SM
 // rather than to what the compiler picks (92 registers, two CTAs as well):
 // the 128 registers that two leave room for let it load a block's rows of B
-// and its values together. Measured (32,768 x 8 random blocks, k = 128): BF16
-// values 193 -> 168 us, FP32 242 -> 186 us, FP64 (16,384 block rows, k = 64)
+// and its values together. Measured (32,768 x 8 random blocks, k = 128, the same
+// B and C again; with three sets in turn BF16 198 -> 178 us): BF16 values
+// 193 -> 168 us, FP32 242 -> 186 us, FP64 (16,384 block rows, k = 64)
 // 152 -> 113 us; three CTAs (80 registers) 187 / 189 / 125 us, one (151)
 // 168 / 260 / 143 us. FP64 B and C with reduced values (FP32 sums, half the
 // accumulators) gain nothing from it (24.6 against 24.9 us, 2,652 x 5 blocks,

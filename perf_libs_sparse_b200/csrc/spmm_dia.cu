@@ -374,14 +374,15 @@ template <> struct DiaPiece<__nv_bfloat16> { using T = uint2; };
 // loop then waits for B's rows alone, once per run, and units that store
 // every entry run without absent checks.
 //
-// Bound by the L1 data pipe (70% of its peak on the 27-point stencil at FP64
+// Bound by the L1 data pipe (74% of its peak on the 27-point stencil at FP64
 // k = 32; B's rows cross it 13.5 times) and by the latency of B's rows.
-// Measured against the kernel above (27-point stencil unless said otherwise):
-// FP64 128^3 k = 32 694 -> 510 us, 80^3 k = 128 527 -> 393 us, 95^3 k = 40
-// 500 -> 352 us, 96^3 k = 16 178 -> 134 us; FP32 128^3 k = 32 256 -> 240 us;
-// BF16 values, 95^3 k = 128 366 -> 320 us; FP64 band of 15, 300,000 rows,
-// k = 64 117 -> 90 us. More CTAs per SM (5 or 6, 48 or 40 registers) or fewer
-// (3) were slower: 811, 751 and 781 us at k = 32.
+// Measured against the kernel above (27-point stencil unless said otherwise;
+// products on the same B and C, with three sets of them in turn 128^3 took
+// 703 -> 549 us): FP64 128^3 k = 32 694 -> 510 us, 80^3 k = 128 527 -> 393 us,
+// 95^3 k = 40 500 -> 352 us, 96^3 k = 16 178 -> 134 us; FP32 128^3 k = 32
+// 256 -> 240 us; BF16 values, 95^3 k = 128 366 -> 320 us; FP64 band of 15,
+// 300,000 rows, k = 64 117 -> 90 us. More CTAs per SM (5 or 6, 48 or 40
+// registers) or fewer (3) were slower: 811, 751 and 781 us at k = 32.
 template <class V, class X, int VEC, class Off>
 __global__ void __launch_bounds__(256, 4)
     k_spmm_dia_staged(int32_t m, int32_t n, int nd, const __grid_constant__ DiaWalk w,

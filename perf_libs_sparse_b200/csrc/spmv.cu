@@ -112,8 +112,9 @@ __device__ __forceinline__ Acc csr_lane_sum(uint32_t j, uint32_t e, const int32_
 // 5.8 us with it first, 4.5 us after the sum, geometric lengths of mean 10 on 4
 // lanes 6.1 and 5.1; equal at 300,000 rows on 4 lanes. First (EARLY) in grids
 // of many waves without the long-row part, whose CTAs even out: 300,000 rows of
-// 0 to 28 entries on 8 lanes 22.8 against 23.1 us, of 40 on 16 lanes 56.1 / 56.7.
-constexpr int64_t kCsrEarlyCtas = 148 * 8 * 6;
+// 0 to 28 entries on 8 lanes 22.8 against 23.1 us, of 40 on 16 lanes 56.1 / 56.7,
+// 354,720 of 8 on 4 lanes (5,542 CTAs) 16.85 / 17.07.
+constexpr int64_t kCsrEarlyCtas = 148 * 8 * 4;
 template <int TPR, bool LONG, bool EARLY, class V, class X>
 __global__ void __launch_bounds__(256)
     k_csr_vector(int32_t m, const int32_t *__restrict__ rp,
@@ -970,16 +971,32 @@ __global__ void __launch_bounds__(256)
   const int e0 = (g % LPB) * W;  // the lane's first value in a block
   const int line = e0 / BS, at = e0 % BS;
   const int i0 = RM ? line : at, j0 = RM ? at : line;
-  uint32_t s = 0, e = 0;  // unsigned: s + step passes 2^31 without overflow
+  const uint32_t step = G / LPB;
+  uint32_t b = 0, b1 = 0;  // unsigned: b + step passes 2^31 without overflow
   if (br < mb) {
-    s = (uint32_t)__ldg(rp + br);
-    e = (uint32_t)__ldg(rp + br + 1);
+    b = (uint32_t)__ldg(rp + br) + g / LPB;
+    b1 = (uint32_t)__ldg(rp + br + 1);
   }
-  const bool big = LONG && e - s > (uint32_t)bsr_long_len(G / LPB);
-  const uint32_t b0 = s + g / LPB, b1 = big ? s : e;
-  int32_t next = b0 < b1 ? __ldg(col + b0) : 0;
+  bool big = false;
+  uint32_t s = 0, e = 0;  // LONG: the block row
+  if constexpr (LONG) {
+    s = br < mb ? b - g / LPB : 0;
+    e = b1;
+    big = e - s > (uint32_t)bsr_long_len(step);
+    if (big)
+      b1 = s;
+  }
+  Acc acc[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+    acc[r] = Acc(0);
+  int32_t next = b < b1 ? __ldg(col + b) : 0;
   const X *x = chain_wait(xg);
-  const auto ld_x = [&](int32_t c, X(&xv)[NC]) {
+  while (b < b1) {
+    const int32_t c = next;
+    V a[W];
+    ld_values(val + (int64_t)b * E + e0, a);
+    X xv[NC];
     if constexpr (XVEC) {
       ld_gather<NC>(x + (int64_t)c * BS + j0, xv);
     } else {
@@ -990,42 +1007,25 @@ __global__ void __launch_bounds__(256)
         xv[j] = one[0];
       }
     }
-  };
-  const auto add_block = [&](const V(&a)[W], const X(&xv)[NC], Acc(&acc)[NR]) {
+    b += step;
+    next = b < b1 ? __ldg(col + b) : 0;
 #pragma unroll
     for (int r = 0; r < NR; ++r)
 #pragma unroll
       for (int j = 0; j < NC; ++j)
         acc[r] = fma(to_acc<Acc>(a[RM ? r * RUN + j : j * RUN + r]), to_acc<Acc>(xv[j]), acc[r]);
-  };
-  // Adds over the lanes of `lanes` that hold the same rows: those of the
-  // block's other columns and of the other lane sets.
-  const auto add_lanes = [&](int lanes, Acc(&acc)[NR]) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const bool rows_differ = o < LPB && (RM ? o * W >= BS : o * W < BS);
-      if (!rows_differ && o < lanes) {
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-          acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-      }
-    }
-  };
-  Acc acc[NR];
-#pragma unroll
-  for (int r = 0; r < NR; ++r)
-    acc[r] = Acc(0);
-  for (uint32_t b = b0; b < b1;) {
-    const int32_t c = next;
-    V a[W];
-    ld_values(val + (int64_t)b * E + e0, a);
-    X xv[NC];
-    ld_x(c, xv);
-    b += G / LPB;
-    next = b < b1 ? __ldg(col + b) : 0;
-    add_block(a, xv, acc);
   }
-  add_lanes(G, acc);
+  // Add over the lanes that hold the same rows: those of the block's other
+  // columns and of the other lane sets.
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const bool rows_differ = o < LPB && (RM ? o * W >= BS : o * W < BS);
+    if (!rows_differ && o < G) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+    }
+  }
   if (br < mb && !big && g < LPB && j0 == 0) {
 #pragma unroll
     for (int r = 0; r < NR; ++r)
@@ -1044,25 +1044,48 @@ __global__ void __launch_bounds__(256)
         acc[r] = Acc(0);
       constexpr int U = BS == 1 ? 8 : 4;  // blocks in flight: nothing else hides the latency
       constexpr uint32_t sets = 32 / LPB;
-      for (uint32_t b = ls + lane / LPB; b < le; b += U * sets) {
+      for (uint32_t p = ls + lane / LPB; p < le; p += U * sets) {
         int32_t c[U];
         V a[U][W];
         X xv[U][NC];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          c[u] = b + u * sets < le ? __ldg(col + b + u * sets) : -1;
+          c[u] = p + u * sets < le ? __ldg(col + p + u * sets) : -1;
 #pragma unroll
         for (int u = 0; u < U; ++u)
           if (c[u] >= 0) {
-            ld_values(val + (int64_t)(b + u * sets) * E + e0, a[u]);
-            ld_x(c[u], xv[u]);
+            ld_values(val + (int64_t)(p + u * sets) * E + e0, a[u]);
+            if constexpr (XVEC) {
+              ld_gather<NC>(x + (int64_t)c[u] * BS + j0, xv[u]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < NC; ++j) {
+                X one[1];
+                ld_gather<1>(x + (int64_t)c[u] * BS + j0 + j, one);
+                xv[u][j] = one[0];
+              }
+            }
           }
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (c[u] >= 0)
-            add_block(a[u], xv[u], acc);
+          if (c[u] >= 0) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+#pragma unroll
+              for (int j = 0; j < NC; ++j)
+                acc[r] = fma(to_acc<Acc>(a[u][RM ? r * RUN + j : j * RUN + r]),
+                             to_acc<Acc>(xv[u][j]), acc[r]);
+          }
       }
-      add_lanes(32, acc);
+#pragma unroll
+      for (int o2 = 1; o2 < 32; o2 <<= 1) {
+        const bool rows_differ = o2 < LPB && (RM ? o2 * W >= BS : o2 * W < BS);
+        if (!rows_differ) {
+#pragma unroll
+          for (int r = 0; r < NR; ++r)
+            acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o2);
+        }
+      }
       if (lane < LPB && j0 == 0) {
 #pragma unroll
         for (int r = 0; r < NR; ++r)
